@@ -48,8 +48,8 @@ WARM_SAMPLE = dict(name="64cubed_same_generator", npart=262_144, nhalo=300, seed
 # instructions, per particle) from the capture summarised in
 # profiles/knn_leaf_kernel_8m.md; the bench line scales them to the workload.
 # They are re-measured whenever the kernel changes.
-NCU_KNN = dict(profiled="knn_leaf_kernel, 8,000,000-particle clustered box, one launch",
-               dram_bytes_per_particle=225.694848, warp_instructions_per_particle=3750.793200)
+NCU_KNN = dict(profiled="knn_collect, knn_finish and knn_query kernels, 8,000,000-particle clustered box, one call",
+               dram_bytes_per_particle=518.172928, warp_instructions_per_particle=1626.264373)
 
 
 def _gen(spec):
@@ -571,7 +571,7 @@ def main():
     achieved = alg / (knn_avg / 1e3) / 1e9
     traffic = NCU_KNN["dram_bytes_per_particle"] * n
     inst = NCU_KNN["warp_instructions_per_particle"]
-    roof = {"kernel": "knn_leaf_kernel", "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+    roof = {"kernel": "knn_collect_kernel + knn_finish_kernel", "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak, "traffic": traffic, "alg_bytes_per_launch": alg,
             "launch_ms": knn_avg, "peak_source": "measured" if peaks else "fallback",
             "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum per particle x n (" +
@@ -602,15 +602,15 @@ def main():
                   "structural_passes": ts[7]}
     nql = max(1, ts[8])
     knn_stats = {"query_leaves": ts[8], "cand_leaves_per_query_leaf": ts[9] / nql,
-                 "leaf_visits_per_query": ts[10] / n, "insertions_per_query": ts[11] / n, "overflow_leaves": ts[12],
-                 "ideal_visits_per_query": ts[18] / n, "chunks_per_query": ts[26] / n,
-                 "ballot_hits_per_query": ts[27] / n,
-                 "union_visits_per_query_leaf": ts[28] / max(1, ts[29]),
-                 "overflow_cycle_share": ts[19] / max(1, ts[19] + ts[20])}
+                 "counted_leaves_per_query_leaf": ts[10] / nql, "collected_per_query": ts[11] / n,
+                 "per_query_search_leaves": ts[12], "per_query_search_queries": ts[18],
+                 "walked_leaves_per_query_leaf": ts[26] / nql, "staged_particles_per_query_leaf": ts[27] / nql,
+                 "rebinned_per_query_leaf": ts[28] / nql,
+                 "per_query_leaf_cycle_share": ts[19] / max(1, ts[19] + ts[20])}
     ph = [float(ts[21 + k]) for k in range(5)]
     if sum(ph) > 0:
         knn_stats["cycle_share"] = {k: v / sum(ph) for k, v in zip(
-            ("bound_and_seed_sort", "candidates_and_sort", "seed_lists", "scan", "density"), ph)}
+            ("bound", "candidates_and_sort", "count", "collect", "order_and_density"), ph)}
     mean_stage = {k: statistics.mean(s[k] for s in stage) for k in
                   ("tree", "knn_density", "hop_groups", "saddles", "nodes", "membership", "total")}
     line = {"metric": METRIC, "value": value, "unit": "Mpart/s", "n_gpus": world, "steps": args.steps,

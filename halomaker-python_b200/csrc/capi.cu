@@ -309,13 +309,13 @@ int ahop_get_timings(AhopTimings* t) {
 
 static void release_device(Engine& E) {
   DevBuf* bufs[] = {&E.d_pos_in, &E.d_mass_in, &E.d_key, &E.d_key2, &E.d_idx, &E.d_idx2, &E.d_x, &E.d_y,
-                    &E.d_z, &E.d_m, &E.d_orig, &E.d_rank, &E.d_box, &E.d_box32, &E.d_cub, &E.d_nei, &E.d_dens,
+                    &E.d_z, &E.d_m, &E.d_p4, &E.d_orig, &E.d_rank, &E.d_box, &E.d_box32, &E.d_cub, &E.d_nei, &E.d_coll, &E.d_dens,
                     &E.d_hop, &E.d_root, &E.d_group, &E.d_peakflag, &E.d_densg, &E.d_gpeak, &E.d_goff,
                     &E.d_gmem, &E.d_gmem_rho, &E.d_gmem_rho_pref, &E.d_sad_key, &E.d_sad_key2, &E.d_sad_val,
                     &E.d_sad_val2, &E.d_sad_cnt, &E.d_sad_keep, &E.d_sad_kpos, &E.d_flags, &E.d_soff,
                     &E.d_sisad, &E.d_srho, &E.d_nodes, &E.d_tree_scratch, &E.d_liste, &E.d_dens_orig,
                     &E.d_rtab, &E.d_itab, &E.d_tprof, &E.d_pairs, &E.d_pair_sums, &E.d_node_aux,
-                    &E.d_forest, &E.d_moff, &E.d_misad, &E.d_mrho, &E.d_kspill, &E.d_task_sort};
+                    &E.d_forest, &E.d_moff, &E.d_misad, &E.d_mrho, &E.d_task_sort};
   if (E.device >= 0) cudaSetDevice(E.device);
   for (DevBuf* b : bufs) b->release();
   E.h_liste.release(); E.h_dens.release(); E.h_rtab.release(); E.h_itab.release();

@@ -102,7 +102,7 @@ struct Engine {
   int32_t forest_rounds = 0, forest_edges = 0;                        // saddle forest of the current compute
   unsigned long long tree_stats[11] = {};                             // structure-tree kernel counters
   unsigned long long knn_stats[12] = {};
-  unsigned long long knn_phase[5] = {};                              // kNN kernel counters
+  unsigned long long knn_phase[5] = {};                              // kNN kernel cycles by phase
   bool events_ready = false;
   AhopTimings timings{};
 
@@ -116,6 +116,7 @@ struct Engine {
   DevBuf d_pos_in, d_mass_in;            // staging for host inputs
   DevBuf d_key, d_key2, d_idx, d_idx2;   // Morton keys + permutation
   DevBuf d_x, d_y, d_z, d_m;             // sorted SoA
+  DevBuf d_p4;                           // the same as (x, y, z, m) rows: one sector per gathered particle
   DevBuf d_orig;                         // orig index (0-based) per sorted slot
   DevBuf d_rank;                         // sorted slot per orig index
   DevBuf d_box;                          // AABBs of all levels (6 doubles each)
@@ -127,7 +128,7 @@ struct Engine {
 
   // kNN / density
   DevBuf d_nei;                          // [n][nstore] sorted-slot neighbour ids
-  DevBuf d_kspill;                       // kNN candidate spill buffers (per resident warp)
+  DevBuf d_coll;                         // collected slots and counts of a chunk of query leaves
   DevBuf d_dens;                         // density in sorted order
   // hop / groups
   DevBuf d_hop, d_root, d_group;         // per sorted slot

@@ -136,20 +136,20 @@ int ahop_debug_compute_stages(const double* pos_in, const double* mass_in, int64
  * (summed over blocks), threshold levels, exact passes for undecided tests,
  * the largest number of levels of one task, the largest cycle count of one
  * task, structural passes; [8..12] kNN -- query leaves, candidate leaves,
- * leaf visits, list insertions, leaves that fell back to per-query search;
- * [13..15] significance tests left undecided by the approximate sums, by
+ * leaves counted, particles collected, query leaves left to the per-query
+ * search; [13..15] significance tests left undecided by the approximate sums, by
  * part: mean density, largest group mean density, densmax or radius;
  * [16..17] saddle forest: Boruvka rounds, forest edges; [18..20] kNN, only
- * while the task profile is on: candidate leaves within each query's final
- * radius, cycles spent in leaves that fell back to per-query search and in
- * the other leaves (summed over warps), then [21..25] the cycles of those
- * other leaves by phase: radius bound, candidate list and its sort, seed
- * lists, candidate scan, density; [26..29] kNN, task profile on: candidate
- * chunks examined, candidate leaves passing a query's box test at its ballot,
- * candidate leaves visited by at least one query of their leaf (leaves whose
- * list stayed in shared memory), and the number of such leaves.  The
- * counters [8..12] and [18..29] come from the profiling instance of the kNN
- * kernel, which runs only while the task profile is on. */
+ * while the task profile is on: queries left to the per-query search, cycles
+ * of the collect kernel in leaves left to it and in the other leaves (summed
+ * over warps), then [21..25] the cycles of those other leaves by phase: radius
+ * bound, candidate lists and their sort, counting scan, collecting scan, and
+ * the finish kernel (exact order and density); [26..29] kNN, task profile on:
+ * listed leaves walked by the two scans, particles staged by them, times a
+ * leaf's bins were laid lower or finer, and 0.  The counters [8..12] and
+ * [18..29] come from the profiling instances of the kNN kernels, which run
+ * only while the task profile is on, and stay 0 for sets small enough for one
+ * warp per query (98,304 particles). */
 int ahop_debug_tree_stats(int64_t* out, int32_t n);
 /* Per-task structure-tree profile (off by default; turning it on costs one
  * store per task).  Row k (32 int64) describes the task of node k (node ids
