@@ -19,7 +19,7 @@
 // potential runs as persistent launches over a work list of (halo, row tile,
 // partner chunk) items sorted by decreasing cost; each item sums m_j / r_ij
 // for its rows over its partners j > i.  Two forms share the schedule:
-//   * FP64: relative positions, 1/r from the double reciprocal square root;
+//   * FP64: relative positions, 1/r in double (pair64.cuh);
 //   * FP32-compensated: positions relative to the halo centre split into
 //     hi = float(r) and lo = float(r - hi) (packed pairs in shared memory);
 //     a pair separation is (hi_j - hi_i) + (lo_j - lo_i) in FP32 (packed
@@ -42,6 +42,7 @@
 
 #include "ahop_halo.h"
 #include "engine.h"
+#include "pair64.cuh"
 
 namespace ahop {
 
@@ -621,7 +622,14 @@ struct PairItem {
   int32_t h, i0, j0, j1;
 };
 
-constexpr int kT64 = 256;  // FP64 form: rows per item = threads per block = partner tile
+constexpr int kT64 = 256;        // FP64 form: rows per item and partner tile
+constexpr int kB64 = 128;        // threads per block: two rows each
+// Partners per item of the FP64 form: as many as leave about kItems64 items
+// (four per resident block), between kMinJ64 and kChunkJ.  With kChunkJ for
+// every call a few large halos left most of the device idle: 217M pairs in 500
+// halos took 2.30 ms as 749 items, 0.19 as 2,333.
+constexpr int64_t kItems64 = 4736;
+constexpr int kMinJ64 = 512;
 
 __device__ __forceinline__ void rel_pos(const HaloArgs& A, int64_t k, double cx, double cy, double cz,
                                         double& rx, double& ry, double& rz) {
@@ -630,13 +638,42 @@ __device__ __forceinline__ void rel_pos(const HaloArgs& A, int64_t k, double cx,
   rz = wrap_chp(A.pos[3 * k + 2] - cz, A.L, A.h, A.periodic);
 }
 
-// Plain FP64 form: relative positions, 1/r from the double reciprocal square
-// root, one row per thread, partner tiles of 256 in shared memory.
-__global__ void __launch_bounds__(kT64) epot64_kernel(HaloArgs A, const PairItem* __restrict__ items,
+// One item of the FP64 form pair by pair as the reference's sum excludes
+// coincident members (r = 0): taken when the fast loops leave a sum that is not
+// finite.  One row per thread and turn.
+__device__ double epot64_careful(const HaloArgs& A, const PairItem& it, int64_t base, int32_t n, double cx, double cy,
+                                 double cz) {
+  double tot = 0.0;
+  for (int32_t i = it.i0 + threadIdx.x; i < min(n, it.i0 + kT64); i += kB64) {
+    double xi, yi, zi, ds = 0.0;
+    rel_pos(A, base + i, cx, cy, cz, xi, yi, zi);
+    for (int32_t j = max(it.j0, i + 1); j < it.j1; ++j) {
+      double x, y, z;
+      rel_pos(A, base + j, cx, cy, cz, x, y, z);
+      const double dx = x - xi, dy = y - yi, dz = z - zi;
+      const double r2 = dx * dx + dy * dy + dz * dz;
+      if (r2 > 0.0) ds += A.mass[base + j] * rsqrt(r2);
+    }
+    tot += A.mass[base + i] * ds;
+  }
+  return tot;
+}
+
+// Plain FP64 form: relative positions, partner tiles of 256 in shared memory
+// as (x, y) and (z, m) rows, two rows per thread.  Bound by the FP64 pipe: 12
+// operations per pair (3 separations, 3 for r^2, 5 for 1/r, 1 for the sum)
+// at 64 per SM and cycle.  A partner's two 16-byte loads serve two rows, and
+// two rows times the unrolled partners are independent chains, where one row
+// per thread and the library's reciprocal square root (13.1 operations) kept
+// the pipe 59 % busy: 6.37e9 pairs in 2,000 halos 9.1 -> 4.84 ms
+// (1.32e12 pairs/s, 85 % of the pipe).
+// Inside the diagonal tile (m members) row i takes the partners i + k mod m,
+// k = 1..m/2, so every pair comes once and no lane waits for another.
+__global__ void __launch_bounds__(kB64) epot64_kernel(HaloArgs A, const PairItem* __restrict__ items,
                                                       int32_t nitems, int32_t* __restrict__ counter,
                                                       double* __restrict__ part) {
-  __shared__ double s_dx[kT64], s_dy[kT64], s_dz[kT64], s_dm[kT64];
-  __shared__ double sh[kT64 / 32];
+  __shared__ __align__(16) double2 s_xy[kT64], s_zm[kT64];
+  __shared__ double sh[kB64 / 32];
   __shared__ int32_t s_item;
   const int tid = threadIdx.x;
   for (;;) {
@@ -650,34 +687,70 @@ __global__ void __launch_bounds__(kT64) epot64_kernel(HaloArgs A, const PairItem
     const int32_t n = (int32_t)(A.off[it.h + 1] - base);
     const double* c = A.out + (size_t)kHaloFields * it.h;
     const double cx = c[HP_PX], cy = c[HP_PY], cz = c[HP_PZ];
-    const int32_t i = it.i0 + tid;
-    const bool vi = i < n;
-    double rxi = 0, ryi = 0, rzi = 0;
-    if (vi) rel_pos(A, base + i, cx, cy, cz, rxi, ryi, rzi);
-    double ds = 0.0;
+    const int32_t rows = min(kT64, n - it.i0);
+    double x0 = -3.0e30, y0 = -3.0e30, z0 = -3.0e30, x1 = -3.0e30, y1 = -3.0e30, z1 = -3.0e30;
+    double m0 = 0.0, m1 = 0.0, d0 = 0.0, d1 = 0.0;
+    if (tid < rows) {
+      rel_pos(A, base + it.i0 + tid, cx, cy, cz, x0, y0, z0);
+      m0 = A.mass[base + it.i0 + tid];
+    }
+    if (tid + kB64 < rows) {
+      rel_pos(A, base + it.i0 + kB64 + tid, cx, cy, cz, x1, y1, z1);
+      m1 = A.mass[base + it.i0 + kB64 + tid];
+    }
+    const bool busy0 = (tid & ~31) < rows, busy1 = (tid & ~31) + kB64 < rows;  // uniform per warp
     for (int32_t j0 = it.j0; j0 < it.j1; j0 += kT64) {
-      const int32_t j = j0 + tid;
-      if (j < it.j1) {
-        double rx, ry, rz;
-        rel_pos(A, base + j, cx, cy, cz, rx, ry, rz);
-        s_dx[tid] = rx; s_dy[tid] = ry; s_dz[tid] = rz; s_dm[tid] = A.mass[base + j];
-      } else {
-        s_dm[tid] = 0.0; s_dx[tid] = s_dy[tid] = s_dz[tid] = 3.0e30;
+      for (int t = tid; t < kT64; t += kB64) {
+        const int32_t j = j0 + t;
+        double rx = 3.0e30, ry = 3.0e30, rz = 3.0e30, m = 0.0;  // past the end: no mass, finite distance
+        if (j < it.j1) {
+          rel_pos(A, base + j, cx, cy, cz, rx, ry, rz);
+          m = A.mass[base + j];
+        }
+        s_xy[t] = make_double2(rx, ry);
+        s_zm[t] = make_double2(rz, m);
       }
       __syncthreads();
-      if (vi) {
-        const int jstart = (j0 == it.i0) ? tid + 1 : 0;  // j > i on the diagonal tile
-        const int jend = min(kT64, it.j1 - j0);
+      const int jend = min(kT64, it.j1 - j0);
+      if (j0 == it.i0) {
+        const int half = (rows - 1) >> 1;  // rows == jend: the halo's or the tile's
+        auto ring = [&](int r, double x, double y, double z, double& d) {
+          int jj = r;
 #pragma unroll 4
-        for (int jj = jstart; jj < jend; ++jj) {
-          const double dx = s_dx[jj] - rxi, dy = s_dy[jj] - ryi, dz = s_dz[jj] - rzi;
-          const double r2 = dx * dx + dy * dy + dz * dz;
-          if (r2 > 0.0) ds += s_dm[jj] * rsqrt(r2);
+          for (int k = 1; k <= half; ++k) {
+            if (++jj == rows) jj = 0;
+            const double2 a = s_xy[jj], b = s_zm[jj];
+            d += b.y * rsqrt3(sep2(a.x - x, a.y - y, b.x - z));
+          }
+          if ((rows & 1) == 0 && r < (rows >> 1)) {
+            const double2 a = s_xy[r + (rows >> 1)], b = s_zm[r + (rows >> 1)];
+            d += b.y * rsqrt3(sep2(a.x - x, a.y - y, b.x - z));
+          }
+        };
+        if (tid < rows) ring(tid, x0, y0, z0, d0);
+        if (tid + kB64 < rows) ring(tid + kB64, x1, y1, z1, d1);
+      } else if (busy1) {
+        const int j4 = (jend + 3) & ~3;
+#pragma unroll 4
+        for (int jj = 0; jj < j4; ++jj) {
+          const double2 a = s_xy[jj], b = s_zm[jj];
+          d0 += b.y * rsqrt3(sep2(a.x - x0, a.y - y0, b.x - z0));
+          d1 += b.y * rsqrt3(sep2(a.x - x1, a.y - y1, b.x - z1));
+        }
+      } else if (busy0) {
+        const int j4 = (jend + 3) & ~3;
+#pragma unroll 4
+        for (int jj = 0; jj < j4; ++jj) {
+          const double2 a = s_xy[jj], b = s_zm[jj];
+          d0 += b.y * rsqrt3(sep2(a.x - x0, a.y - y0, b.x - z0));
         }
       }
       __syncthreads();
     }
-    const double tot = block_sum(vi ? A.mass[base + i] * ds : 0.0, sh);
+    double tot = m0 * d0 + m1 * d1;
+    // a coincident pair leaves inf or NaN in its row
+    if (__syncthreads_or(!(fabs(tot) <= DBL_MAX))) tot = epot64_careful(A, it, base, n, cx, cy, cz);
+    tot = block_sum<double, kB64>(tot, sh);
     if (tid == 0) part[w] = tot;
   }
 }
@@ -1243,13 +1316,13 @@ struct ItemList {
 };
 
 // Items of halo h (n members) with `rows` rows per item over rows [0, row_limit),
-// partners in chunks of kChunkJ.
-static void add_halo_items(ItemList& L, int32_t h, int64_t n, int rows, int64_t row_limit) {
+// partners in chunks of `chunk`, a multiple of the row count.
+static void add_halo_items(ItemList& L, int32_t h, int64_t n, int rows, int64_t row_limit, int64_t chunk = kChunkJ) {
   const int64_t rl = std::min(n, row_limit);
   for (int64_t i0 = 0; i0 < rl; i0 += rows) {
     const int64_t r = std::min<int64_t>(rows, n - i0);
-    for (int64_t j0 = i0; j0 < n; j0 += kChunkJ) {
-      const int64_t j1 = std::min<int64_t>(n, j0 + kChunkJ);
+    for (int64_t j0 = i0; j0 < n; j0 += chunk) {
+      const int64_t j1 = std::min<int64_t>(n, j0 + chunk);
       L.items.push_back(PairItem{h, (int32_t)i0, (int32_t)j0, (int32_t)j1});
       L.cost.push_back(j0 == i0 ? r * (j1 - j0) - r * r / 2 : r * (j1 - j0));
     }
@@ -1497,7 +1570,7 @@ static int enqueue_props(HaloEngine& H, const HaloArgs& A, int64_t nhalo, int ep
   }
   AHOP_CUDA_TRY(cudaEventRecordWithFlags(H.ev[1], s, flags));
   if ((epot & 1) && H.l64.n > 0) {
-    epot64_kernel<<<grid64, kT64, 0, s>>>(A, H.l64.items.as<PairItem>(), H.l64.n, H.d_counter.as<int32_t>(),
+    epot64_kernel<<<grid64, kB64, 0, s>>>(A, H.l64.items.as<PairItem>(), H.l64.n, H.d_counter.as<int32_t>(),
                                           H.l64.part.as<double>());
     ++*launches;
     AHOP_CUDA_TRY(cudaGetLastError());
@@ -1593,6 +1666,8 @@ static int halo_run(HaloEngine& H, const AhopHaloParams* p, const int64_t* d_off
     }
   }
   // work lists (halo order), schedules, per-halo shape codes
+  const int64_t fit64 = (int64_t)(pairs / ((double)kItems64 * kT64));
+  const int64_t chunk64 = std::min<int64_t>(kChunkJ, std::max<int64_t>(kMinJ64, (fit64 + kT64 - 1) / kT64 * kT64));
   std::vector<int8_t> hshape;
   H.L64.clear();
   H.L32.clear();
@@ -1603,7 +1678,7 @@ static int halo_run(HaloEngine& H, const AhopHaloParams* p, const int64_t* d_off
     const int64_t n = h_off[h + 1] - h_off[h];
     H.L64.hoff[h] = (int64_t)H.L64.items.size();
     H.L32.hoff[h] = (int64_t)H.L32.items.size();
-    if (epot & 1) add_halo_items(H.L64, (int32_t)h, n, kT64, n);
+    if (epot & 1) add_halo_items(H.L64, (int32_t)h, n, kT64, n, chunk64);
     if (epot & 2) {
       const int b = bucket_of(n);
       const int c = H.pinned[b] >= 0 ? H.pinned[b] : H.code[b] >= 0 ? H.code[b] : kDefaultShape;
@@ -1622,7 +1697,7 @@ static int halo_run(HaloEngine& H, const AhopHaloParams* p, const int64_t* d_off
   if ((rc = upload_list(H.l64, H.L64, st))) return rc;
   if ((rc = upload_list(H.l32, H.L32, st))) return rc;
   if ((rc = upload(H.d_hshape, hshape, st))) return rc;
-  const int grid64 = grid_for((const void*)epot64_kernel, kT64);
+  const int grid64 = grid_for((const void*)epot64_kernel, kB64);
   const int grid32 = grid_for((const void*)epot32_kernel, kB32);
   // the launches run on the engine's stream after everything queued on st
   AHOP_CUDA_TRY(cudaEventRecord(H.ev_in, st));
@@ -1941,7 +2016,7 @@ extern "C" int ahop_halo_props_noalloc(const AhopHaloParams* p, const int64_t* d
   halo_moments_kernel<<<(unsigned)nhalo, kPB, 0, st>>>(A);
   AHOP_CUDA_TRY(cudaGetLastError());
   if ((p->epot & 1) && total > 0) {
-    epot64_kernel<<<grid_for((const void*)epot64_kernel, kT64), kT64, 0, st>>>(A, S->items, total, &S->counter[0],
+    epot64_kernel<<<grid_for((const void*)epot64_kernel, kB64), kB64, 0, st>>>(A, S->items, total, &S->counter[0],
                                                                                S->part64);
     AHOP_CUDA_TRY(cudaGetLastError());
   }
