@@ -339,6 +339,7 @@ int ahop_close(void) {
 }
 
 int ahop_release_device_memory(void) {
+  release_adjoint_memory();
   if (!g_engine) return AHOP_OK;
   ahop_close();
   release_device(*g_engine);

@@ -65,3 +65,34 @@ def test_pairs_over_the_range_of_separations():
     mass = np.tile([2.0, 1.0], 4000)  # the denser member, at the origin, is the centre
     got = _ep64(np.arange(0, 8001, 2), pos, mass, periodic=False)
     assert np.all(np.abs(got * d + 2.0) <= 2.0 * 4 * 2.0 ** -52)
+
+
+@pytest.mark.parametrize("coincident", [False, True])
+def test_gradient_at_tile_edges(coincident):
+    import torch
+    from ahop_b200 import autograd
+    rng = np.random.default_rng(9)
+    sizes = SIZES + [5000]  # partners of the largest go to ten items
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    pos = rng.normal(size=(off[-1], 3))
+    mass = rng.uniform(0.5, 1.5, off[-1])
+    if coincident:
+        for a, b in zip(off[:-1], off[1:]):
+            if b - a > 2:
+                pos[b - 1] = pos[a]
+                pos[a + (b - a) // 2] = pos[a]
+    dev = torch.device("cuda:0")
+    gh = rng.normal(size=len(sizes))
+    p = torch.from_numpy(pos).to(dev).requires_grad_(True)
+    e = autograd.HaloPotential.apply(p, torch.from_numpy(mass).to(dev), torch.from_numpy(off), 100.0, 1.0)
+    e.backward(torch.from_numpy(gh).to(dev))
+    grad = p.grad.cpu().numpy()
+    for h, (a, b) in enumerate(zip(off[:-1], off[1:])):
+        x, m = pos[a:b], mass[a:b]
+        for i in rng.choice(b - a, min(b - a, 300), replace=False):
+            d = x[i] - x
+            r2 = (d * d).sum(1)
+            w = m / np.where(r2 > 0, r2, np.inf) ** 1.5
+            terms = gh[h] * m[i] * w[:, None] * d
+            # each term within 1e-13 (separations of positions rounded once), n terms
+            assert np.all(np.abs(grad[a + i] - terms.sum(0)) <= 1e-12 * np.abs(terms).sum(0) + 1e-300), (b - a, i)
