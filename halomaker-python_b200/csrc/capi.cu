@@ -340,6 +340,7 @@ int ahop_close(void) {
 
 int ahop_release_device_memory(void) {
   release_adjoint_memory();
+  release_reader_memory();
   if (!g_engine) return AHOP_OK;
   ahop_close();
   release_device(*g_engine);

@@ -180,7 +180,8 @@ int stage_knn_density(Engine& E);
 int stage_hop_groups(Engine& E);
 int stage_saddles(Engine& E);
 int stage_nodes(Engine& E);
-void release_adjoint_memory();  // workspace of the potential's gradient (adjoint.cu)
+void release_adjoint_memory();  // workspaces of the gradients (adjoint.cu)
+void release_reader_memory();   // staging of the part-file reader (ramses.cu)
 int build_saddle_forest(Engine& E);  // maximum spanning forest of the saddle rows (forest.cu)
 
 }  // namespace ahop
