@@ -12,9 +12,10 @@
 //
 // Order.  GL keeps the reference's igr order (f90:1337-1367): components are
 // contiguous, ordered by their smallest position before the level, and keep
-// their previous relative order inside.  Components are found with a
-// block-level union-find over saddle edges > rhot linking to the smaller
-// position, then reordered by a chunked stable radix sort on the root.  The
+// their previous relative order inside.  Components are found over the saddle
+// edges > rhot (listed once per task) with labels or a union-find that link to
+// the smaller position, then reordered by a chunked stable radix sort on the
+// root.  The
 // structure can only change when rhot crosses a saddle value or a group peak
 // density of the task, so this pass is skipped at levels below the next such
 // value.
@@ -71,6 +72,13 @@ struct Task {
   int32_t inode, a, b, level;
 };
 
+// An edge of the saddle forest inside a task's range, listed by the task's
+// first structural pass.
+struct __align__(16) EdgeRec {
+  int32_t u, v;  // groups
+  double w;      // saddle
+};
+
 struct TreeArgs {
   // particles (sorted order)
   const double *x, *y, *z, *m, *dens;
@@ -102,9 +110,11 @@ struct TreeArgs {
   int32_t* cstart;        // [ng] component k of a task starts at cstart[a+k]
   int32_t* compidx;       // [ng] component index of each position
   int32_t* gn;            // [ng] per-position member count above rhot
-  double* gs;             // [ng][8] per-position scratch sums
+  double* gs;             // [8][ng+1] per-position scratch sums, value by value (a warp's positions are neighbours)
   double* cs;             // [ng][12] per-component scratch
   int32_t* deepnode;      // [ng+1]
+  EdgeRec* elist;         // [ng] edges of the task whose range starts at position a: [a, a + ecnt[a])
+  int32_t* ecnt;          // [ng]
   int32_t* gcur;          // [ng+1] members above the group's last threshold
   int32_t* ecur;          // [ng+1] saddle-row entries above the group's last threshold
   NodeRec* node;          // [nnodesmax+1]
@@ -129,6 +139,8 @@ struct TreeArgs {
   unsigned long long* stats;  // [11] counters (see the end of tree_wave_kernel; [8..10] undecided tests)
   long long* tprof;       // [nnodesmax+1][kProfRow] per-task profile row by node id, or null
 };
+
+__device__ __forceinline__ size_t gs_stride(const TreeArgs& A) { return (size_t)A.ngroups + 1; }
 
 __device__ __forceinline__ void set_err(const TreeArgs& A, int code, int detail) {
   if (atomicCAS(A.err, 0, code) == 0) A.err[1] = detail;
@@ -193,20 +205,36 @@ __device__ __forceinline__ int32_t count_above_at(const TreeArgs& A, int32_t g, 
                                                   double rhot) {
   if (hi == 0 || rlast > rhot) return hi;
   const double* r = A.rdesc + off;
-  // r[j] <= rhot; gallop down until an index above rhot (or 0) brackets the answer
-  int32_t j = hi - 1, lo = 0, step = 1;
-  while (true) {
-    const int32_t k = j - step;
-    if (k < 0) { lo = 0; break; }
-    if (r[k] > rhot) { lo = k + 1; break; }
-    j = k;
-    step <<= 1;
+  // r[j] <= rhot.  Eight probes at growing distances below j at once, then
+  // seven inside the bracket at once: every round's loads are independent
+  // (one at a time they were a chain of about ten memory latencies per level).
+  int32_t j = hi - 1, lo = -1;
+  while (lo < 0) {
+    double v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = j - (1 << k) >= 0 ? r[j - (1 << k)] : DBL_MAX;
+    int k = 0;
+#pragma unroll
+    for (int t = 7; t >= 0; --t) k = v[t] > rhot ? t : k;  // the nearest probe above rhot
+    if (v[7] > rhot) {
+      lo = max(0, j - (1 << k) + 1);
+      if (k > 0) j -= 1 << (k - 1);
+    } else {
+      j -= 128;
+    }
   }
-  int32_t a2 = lo, b2 = j;  // first index with r <= rhot lies in [lo, j]
-  while (a2 < b2) {
-    const int32_t mid = (a2 + b2) >> 1;
-    if (r[mid] > rhot) a2 = mid + 1; else b2 = mid;
+  while (lo < j) {  // first index with r <= rhot lies in [lo, j]
+    const int32_t len = j - lo;
+    int32_t above = lo;  // after the last probe above rhot
+#pragma unroll
+    for (int k = 0; k < 7; ++k) {
+      const int32_t i = lo + (int32_t)(((int64_t)len * (k + 1)) >> 3);
+      if (r[i] > rhot) above = i + 1;
+      else j = min(j, i);
+    }
+    lo = above;
   }
+  const int32_t a2 = lo;
   A.gcur[g] = a2;
   return a2;
 }
@@ -295,6 +323,7 @@ struct SharedTask {
   int32_t phase, plocal;
   double ev_part[kClusterCtas];
   int32_t fold_n;  // large components whose partial sums a decide phase folds
+  int32_t nedges;  // edges listed for the task (-1: the next structural pass lists them)
 };
 
 namespace cg = cooperative_groups;
@@ -316,6 +345,16 @@ __device__ __forceinline__ void lead_phase(SharedTask& T, int32_t code, bool loc
 // CTAs (see tree_wave_kernel).  par is the union-find array (entries relative
 // to poff), in the leader CTA's shared memory or in global memory.
 //
+// A task's first pass lists the forest edges above its threshold (fewer than
+// its groups: a forest); later ones come from the list.
+__device__ __forceinline__ void list_edge(const TreeArgs& A, int32_t a, int32_t b, int32_t u, int32_t v, double w) {
+  const int32_t s = atomicAdd(&A.ecnt[a], 1);
+  if (s >= b - a) { set_err(A, 19, u); return; }
+  EdgeRec r;
+  r.u = u; r.v = v; r.w = w;
+  A.elist[a + s] = r;
+}
+
 // Union over saddle edges above rhot (a prefix of each row, rows sorted by
 // decreasing saddle).  Each undirected edge is linked once, from the row of
 // its smaller group id; rows with more than kRowWarp such edges go to the
@@ -344,7 +383,10 @@ __device__ void union_short_rows(const TreeArgs& A, int32_t a, int32_t b, int32_
       const int32_t h = A.sisad[e];
       const int32_t j = A.pos_of[h];
       if (j < a || j >= b) { set_err(A, 11, g); continue; }  // f90:1229-1233
-      if (h > g) uf_union(par, i - poff, j - poff);
+      if (h > g) {
+        list_edge(A, a, b, g, h, A.srho[e]);
+        uf_union(par, i - poff, j - poff);
+      }
     }
   }
 #pragma unroll
@@ -366,7 +408,99 @@ __device__ void union_long_rows(const TreeArgs& A, int32_t a, int32_t b, int32_t
       const int32_t h = A.sisad[e];
       const int32_t j = A.pos_of[h];
       if (j < a || j >= b) { set_err(A, 11, g); continue; }
-      if (h > g) uf_union(par, i - poff, j - poff);
+      if (h > g) {
+        list_edge(A, a, b, g, h, A.srho[e]);
+        uf_union(par, i - poff, j - poff);
+      }
+    }
+  }
+}
+
+// The same union from the task's edge list, one edge per thread: the rows'
+// chain of dependent loads per group (cursor, last saddle, search, neighbour,
+// its position) is paid once per task.  A pruned group's edges stay listed; its
+// position is -1.  For tasks whose parents are in global memory.
+template <int NT>
+__device__ void union_edges(const TreeArgs& A, int32_t a, int32_t b, int32_t ne, int32_t poff, double rhot,
+                            int32_t* par, double* ev_min, int32_t gt, int32_t gs) {
+  double ev = DBL_MAX;
+  for (int32_t i = a + gt; i < b; i += gs) {
+    const double dg = A.densg[A.GL[i]];
+    if (dg > rhot) ev = fmin(ev, dg);
+  }
+  for (int32_t e = gt; e < ne; e += gs) {
+    const EdgeRec r = A.elist[a + e];
+    if (!(r.w > rhot)) continue;
+    const int32_t pu = A.pos_of[r.u], pv = A.pos_of[r.v];
+    if (pu < 0 || pv < 0) continue;
+    ev = fmin(ev, r.w);
+    if (pu < a || pu >= b || pv < a || pv >= b) { set_err(A, 11, r.u); continue; }
+    uf_union(par, pu - poff, pv - poff);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ev = fmin(ev, __shfl_xor_sync(0xffffffffu, ev, o));
+  if ((threadIdx.x & 31) == 0 && ev < DBL_MAX) atomic_min_pos(ev_min, ev);
+}
+
+// Component labels of a task whose parents are in the block's shared memory,
+// from its edge list: every edge between two labels hooks the larger under the
+// smaller, then all labels are followed to their ends, until no edge joins two
+// labels (two to five rounds).  The same labels as the unions', the smallest
+// position of each component, without their compare-and-swap chains; a wide
+// task's leader does it alone.  s_edge holds the edges' positions, packed.
+// A level of a 496-group task (262,144-particle box, 74 levels), cycles: union
+// and roots 21,500 -> 8,600 (bound by the latency of the position and density
+// loads), group terms 10,000 -> 7,300 (probes below the cursor at once), whole
+// level 52,600 -> 40,900; structure-tree waves, ms: 262,144 particles 2.34 ->
+// 1.83, 2M 3.35 -> 2.82, 16.7M 7.18 -> 6.52.
+template <int NT>
+__device__ void label_edges(const TreeArgs& A, int32_t a, int32_t b, int32_t ne, double rhot, int32_t* par,
+                            int32_t* s_edge, int32_t cap, double* ev_min) {
+  const int tid = threadIdx.x;
+  int32_t* edge = ne <= cap ? s_edge : A.GL2 + a;  // GL2: free until the reorder
+  double ev = DBL_MAX;
+  for (int32_t i = a + tid; i < b; i += NT) {
+    const double dg = A.densg[A.GL[i]];
+    if (dg > rhot) ev = fmin(ev, dg);
+  }
+  bool open = false;
+  for (int32_t e = tid; e < ne; e += NT) {
+    const EdgeRec r = A.elist[a + e];
+    int32_t pk = -1;
+    if (r.w > rhot) {
+      const int32_t pu = A.pos_of[r.u], pv = A.pos_of[r.v];
+      if (pu >= 0 && pv >= 0) {
+        ev = fmin(ev, r.w);
+        if (pu < a || pu >= b || pv < a || pv >= b) set_err(A, 11, r.u);
+        else {
+          const int32_t lo = min(pu, pv) - a, hi = max(pu, pv) - a;
+          pk = lo | (hi << 16);  // below 32,768: the shared array's limit
+          atomicMin(&par[hi], lo);
+          open = true;
+        }
+      }
+    }
+    edge[e] = pk;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ev = fmin(ev, __shfl_xor_sync(0xffffffffu, ev, o));
+  if ((tid & 31) == 0 && ev < DBL_MAX) atomic_min_pos(ev_min, ev);
+  while (__syncthreads_or(open)) {
+    for (int32_t i = tid; i < b - a; i += NT) {
+      int32_t r = par[i];
+      for (int32_t q = par[r]; q != r; q = par[r]) r = q;
+      par[i] = r;
+    }
+    __syncthreads();
+    open = false;
+    for (int32_t e = tid; e < ne; e += NT) {
+      const int32_t pk = edge[e];
+      if (pk < 0) continue;
+      const int32_t u = par[pk & 0xffff], v = par[pk >> 16];
+      if (u != v) {
+        atomicMin(&par[max(u, v)], min(u, v));
+        open = true;
+      }
     }
   }
 }
@@ -508,7 +642,12 @@ __device__ void structural_pass(const TreeArgs& A, SharedTask& T, typename SortT
   auto mark = [&](int k) {
     if (tid == 0) { const long long t = clock64(); ph[k] += t - tl; tl = t; }
   };
-  if (tid == 0) { T.next_event = DBL_MAX; T.nbig = 0; }
+  const int32_t ne = T.nedges;
+  if (tid == 0) {
+    T.next_event = DBL_MAX;
+    T.nbig = 0;
+    if (ne < 0) A.ecnt[a] = 0;
+  }
   for (int32_t i = a + tid; i < b; i += NT) {
     par[i - poff] = i - poff;
     A.cnt[i] = 0;
@@ -517,17 +656,25 @@ __device__ void structural_pass(const TreeArgs& A, SharedTask& T, typename SortT
   __syncthreads();
   mark(0);
   const int K = NT >= 1024 ? cluster_ctas() : 1;
-  if (K > 1) lead_phase(T, kPhUnion, local);
-  union_short_rows<NT>(A, a, b, poff, rhot, par, s_big, &T.nbig, &T.next_event, tid, K * NT);
-  __syncthreads();
-  mark(12);
-  union_long_rows<NT>(A, a, b, poff, par, s_big, T.nbig);
-  if (K > 1) {
+  const bool label = ne >= 0 && local;
+  if (K > 1 && !label) lead_phase(T, kPhUnion, local);
+  if (label) {
+    label_edges<NT>(A, a, b, ne, rhot, par, s_keys, NT * IPT, &T.next_event);
+  } else if (ne < 0) {
+    union_short_rows<NT>(A, a, b, poff, rhot, par, s_big, &T.nbig, &T.next_event, tid, K * NT);
+    __syncthreads();
+    mark(12);
+    union_long_rows<NT>(A, a, b, poff, par, s_big, T.nbig);
+  } else {
+    union_edges<NT>(A, a, b, ne, poff, rhot, par, &T.next_event, tid, K * NT);
+  }
+  if (K > 1 && !label) {
     cg::this_cluster().sync();  // the followers' unions and next events are in
     if (tid == 0)
       for (int r = 1; r < K; ++r) T.next_event = fmin(T.next_event, T.ev_part[r]);
   }
   __syncthreads();
+  if (ne < 0 && tid == 0) T.nedges = min(atomicAdd(&A.ecnt[a], 0), b - a);
   mark(1);
   if (K > 1) lead_phase(T, kPhFind, local);
   find_roots(A, a, b, poff, rhot, par, tid, K * NT);
@@ -643,7 +790,8 @@ __device__ __forceinline__ int tri_gt(double v, double t, double e) {
 __device__ __forceinline__ void store_terms(const TreeArgs& A, int32_t i, int32_t ng, double dg, const double* P,
                                             double dx, double dy, double dz, double rhot) {
   const double u = 1.1102230246251565e-16;
-  double* G = A.gs + 8 * (size_t)i;
+  double* G = A.gs + i;
+  const size_t S = gs_stride(A);
   A.gn[i] = ng;
   double t[7] = {0, 0, 0, 0, 0, 0, (double)kFalse};
   if (ng > 0) {
@@ -660,7 +808,7 @@ __device__ __forceinline__ void store_terms(const TreeArgs& A, int32_t i, int32_
   }
   G[0] = dg;
 #pragma unroll
-  for (int c = 0; c < 7; ++c) G[1 + c] = t[c];
+  for (int c = 0; c < 7; ++c) G[(1 + c) * S] = t[c];
 }
 
 __device__ __forceinline__ void position_terms(const TreeArgs& A, int32_t i, double rhot, const double* a) {
@@ -731,19 +879,20 @@ __device__ void component_decide_thread(const TreeArgs& A, int32_t c0, int32_t c
   int32_t nmax = 0;
   double dmax = -1.0, S = 0, M = 0, Sx = 0, Sy = 0, Sz = 0, Q = 0;
   int triB = kFalse;
+  const size_t gst = gs_stride(A);
   for (int32_t i = c0; i < c1; ++i) {
-    const double* G = A.gs + 8 * (size_t)i;
+    const double* G = A.gs + i;
     const int32_t ng = A.gn[i];
     nl += ng;
     nmax = max(nmax, ng);
     dmax = fmax(dmax, G[0]);
-    S += G[1];
-    M += G[2];
-    Sx += G[3];
-    Sy += G[4];
-    Sz += G[5];
-    Q += G[6];
-    triB = tri_or(triB, (int)G[7]);
+    S += G[1 * gst];
+    M += G[2 * gst];
+    Sx += G[3 * gst];
+    Sy += G[4 * gst];
+    Sz += G[5 * gst];
+    Q += G[6 * gst];
+    triB = tri_or(triB, (int)G[7 * gst]);
   }
   decide_from_sums(A, rhot, nl, nmax, dmax, S, M, Sx, Sy, Sz, Q, triB, C);
 }
@@ -753,20 +902,21 @@ __device__ void component_decide(const TreeArgs& A, int32_t c0, int32_t c1, doub
   int32_t nmax = 0;
   double dmax = -1.0, S = 0, M = 0, Sx = 0, Sy = 0, Sz = 0, Q = 0;
   int triB = kFalse;  // densmoy_comp_max > rhot
+  const size_t gst = gs_stride(A);
 #pragma unroll 4
   for (int32_t i = c0 + lane; i < c1; i += 32) {
-    const double* G = A.gs + 8 * (size_t)i;
+    const double* G = A.gs + i;
     const int32_t ng = A.gn[i];
     nl += ng;
     nmax = max(nmax, ng);
     dmax = fmax(dmax, G[0]);
-    S += G[1];
-    M += G[2];
-    Sx += G[3];
-    Sy += G[4];
-    Sz += G[5];
-    Q += G[6];
-    triB = tri_or(triB, (int)G[7]);
+    S += G[1 * gst];
+    M += G[2 * gst];
+    Sx += G[3 * gst];
+    Sy += G[4 * gst];
+    Sz += G[5 * gst];
+    Q += G[6 * gst];
+    triB = tri_or(triB, (int)G[7 * gst]);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -799,20 +949,21 @@ __device__ CompSums block_partial_sums(const TreeArgs& A, int32_t c0, int32_t c1
                                        CompSums* red) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   CompSums s{0, 0, kFalse, -1.0, 0, 0, 0, 0, 0, 0};
+  const size_t gst = gs_stride(A);
 #pragma unroll 4
   for (int32_t i = c0 + gt; i < c1; i += gs) {
-    const double* G = A.gs + 8 * (size_t)i;
+    const double* G = A.gs + i;
     const int32_t ng = A.gn[i];
     s.nl += ng;
     s.nmax = max(s.nmax, ng);
     s.dmax = fmax(s.dmax, G[0]);
-    s.S += G[1];
-    s.M += G[2];
-    s.Sx += G[3];
-    s.Sy += G[4];
-    s.Sz += G[5];
-    s.Q += G[6];
-    s.triB = tri_or(s.triB, (int)G[7]);
+    s.S += G[1 * gst];
+    s.M += G[2 * gst];
+    s.Sx += G[3 * gst];
+    s.Sy += G[4 * gst];
+    s.Sz += G[5 * gst];
+    s.Q += G[6 * gst];
+    s.triB = tri_or(s.triB, (int)G[7 * gst]);
   }
   auto fold = [&](CompSums& v) {
 #pragma unroll
@@ -982,7 +1133,7 @@ __device__ void approx_stats(const TreeArgs& A, SharedTask& T, long long* ph, in
 // unwrapped about posref then shifted back.  G[0..6] = imass, truemass,
 // posg(3), rsquare, densmoy.
 __device__ void group_sums_thread(const TreeArgs& A, int32_t g, double rhot, double rx, double ry, double rz,
-                                  double* G) {
+                                  double* G, size_t st) {
   int32_t imass = 0;
   double tm = 0, px = 0, py = 0, pz = 0, rs = 0, dm = 0;
   for (int32_t q = A.goff[g]; q < A.goff[g + 1]; ++q) {
@@ -1004,7 +1155,7 @@ __device__ void group_sums_thread(const TreeArgs& A, int32_t g, double rhot, dou
     rs = xadd(rs, xmul(xm, xadd(xadd(xmul(ux, ux), xmul(uy, uy)), xmul(uz, uz))));
     dm = xadd(dm, d);
   }
-  G[0] = (double)imass; G[1] = tm; G[2] = px; G[3] = py; G[4] = pz; G[5] = rs; G[6] = dm;
+  G[0] = (double)imass; G[st] = tm; G[2 * st] = px; G[3 * st] = py; G[4 * st] = pz; G[5 * st] = rs; G[6 * st] = dm;
 }
 
 // Same sums for a large group by one warp: each lane computes the terms of
@@ -1014,7 +1165,7 @@ __device__ void group_sums_thread(const TreeArgs& A, int32_t g, double rhot, dou
 // roundings as the Fortran loop, without one dependent global load per
 // member on one thread.  st: 32*6 doubles of warp-private shared memory.
 __device__ void group_sums_warp(const TreeArgs& A, int32_t g, double rhot, double rx, double ry, double rz,
-                                double* G, double* st, int lane) {
+                                double* G, size_t gst, double* st, int lane) {
   const int32_t q0 = A.goff[g], q1 = A.goff[g + 1];
   int32_t imass = 0;
   double acc = 0.0;  // lane c < 6 carries sum c: truemass, posg(3), rsquare, densmoy
@@ -1060,7 +1211,9 @@ __device__ void group_sums_warp(const TreeArgs& A, int32_t g, double rhot, doubl
   const double pz = __shfl_sync(0xffffffffu, acc, 3);
   const double rs = __shfl_sync(0xffffffffu, acc, 4);
   const double dm = __shfl_sync(0xffffffffu, acc, 5);
-  if (lane == 0) { G[0] = (double)imass; G[1] = tm; G[2] = px; G[3] = py; G[4] = pz; G[5] = rs; G[6] = dm; }
+  if (lane == 0) {
+    G[0] = (double)imass; G[gst] = tm; G[2 * gst] = px; G[3 * gst] = py; G[4 * gst] = pz; G[5 * gst] = rs; G[6 * gst] = dm;
+  }
 }
 
 // posref of a colour: first particle above rhot of its first group (f90:2340-2344).
@@ -1079,21 +1232,22 @@ __device__ int32_t colour_posref(const TreeArgs& A, int32_t g0, double rhot) {
 __device__ void colour_fold(const TreeArgs& A, int32_t c0, int32_t c1, double rhot, double* C) {
   double posg0 = 0, posg1 = 0, posg2 = 0, tm = 0, rsg = 0, dmg = 0, dmax = -1.0, dcm = -1.0;
   int32_t ml = 0, mc = 0;
+  const size_t gst = gs_stride(A);
   for (int32_t i = c0; i < c1; ++i) {
-    const double* G = A.gs + 8 * (size_t)i;
+    const double* G = A.gs + i;
     const int32_t g = A.GL[i];
     dmax = fmax(dmax, A.densg[g]);
     const int32_t mt = (int32_t)G[0];
-    posg0 = xadd(posg0, G[2]);
-    posg1 = xadd(posg1, G[3]);
-    posg2 = xadd(posg2, G[4]);
-    rsg = xadd(rsg, G[5]);
+    posg0 = xadd(posg0, G[2 * gst]);
+    posg1 = xadd(posg1, G[3 * gst]);
+    posg2 = xadd(posg2, G[4 * gst]);
+    rsg = xadd(rsg, G[5 * gst]);
     ml += mt;
-    tm = xadd(tm, G[1]);
-    dmg = xadd(dmg, G[6]);
+    tm = xadd(tm, G[1 * gst]);
+    dmg = xadd(dmg, G[6 * gst]);
     mc = max(mc, mt);
     if (mt > 0) {
-      const double dmt = xdiv(G[6], (double)mt);
+      const double dmt = xdiv(G[6 * gst], (double)mt);
       dcm = fmax(dcm, xdiv(dmt, xadd(1.0, xdiv(A.fudge, xsqrt((double)mt)))));
     }
   }
@@ -1125,7 +1279,7 @@ __device__ void exact_stats(const TreeArgs& A, SharedTask& T, double* s_terms) {
     const int32_t g = A.GL[i];
     if (A.goff[g + 1] - A.goff[g] <= kBigGroup) continue;
     const int32_t ref = (int32_t)C[11];
-    group_sums_warp(A, g, rhot, A.x[ref], A.y[ref], A.z[ref], A.gs + 8 * (size_t)i, s_terms + warp * 32 * 6, lane);
+    group_sums_warp(A, g, rhot, A.x[ref], A.y[ref], A.z[ref], A.gs + i, gs_stride(A), s_terms + warp * 32 * 6, lane);
   }
   for (int32_t i = T.a + tid; i < T.b; i += NT) {  // small groups: a thread each
     const double* C = A.cs + 12 * (size_t)(T.a + A.compidx[i]);
@@ -1133,7 +1287,7 @@ __device__ void exact_stats(const TreeArgs& A, SharedTask& T, double* s_terms) {
     const int32_t g = A.GL[i];
     if (A.goff[g + 1] - A.goff[g] > kBigGroup) continue;
     const int32_t ref = (int32_t)C[11];
-    group_sums_thread(A, g, rhot, A.x[ref], A.y[ref], A.z[ref], A.gs + 8 * (size_t)i);
+    group_sums_thread(A, g, rhot, A.x[ref], A.y[ref], A.z[ref], A.gs + i, gs_stride(A));
   }
   __syncthreads();
   for (int32_t k = tid; k < T.ncomp; k += NT) {
@@ -1243,11 +1397,11 @@ __global__ void __launch_bounds__(kNT) root_colour_kernel(const TreeArgs A, int3
   for (int32_t i = c0 + warp; i < c1; i += kNT / 32) {
     const int32_t g = A.GL[i];
     if (A.goff[g + 1] - A.goff[g] > kBigGroup)
-      group_sums_warp(A, g, rhot, rx, ry, rz, A.gs + 8 * (size_t)i, s_terms + warp * 32 * 6, lane);
+      group_sums_warp(A, g, rhot, rx, ry, rz, A.gs + i, gs_stride(A), s_terms + warp * 32 * 6, lane);
   }
   for (int32_t i = c0 + tid; i < c1; i += kNT) {
     const int32_t g = A.GL[i];
-    if (A.goff[g + 1] - A.goff[g] <= kBigGroup) group_sums_thread(A, g, rhot, rx, ry, rz, A.gs + 8 * (size_t)i);
+    if (A.goff[g + 1] - A.goff[g] <= kBigGroup) group_sums_thread(A, g, rhot, rx, ry, rz, A.gs + i, gs_stride(A));
   }
   __syncthreads();
   if (tid == 0) colour_fold(A, c0, c1, rhot, A.cs + 12 * (size_t)k);
@@ -1358,10 +1512,12 @@ __device__ void prune_low_components(const TreeArgs& A, SharedTask& T, typename 
   for (int32_t i = a + tid; i < b; i += NT) {
     const int32_t k = A.compidx[i];
     const int32_t g = A.GL[i];
-    if (A.cs[12 * (size_t)(a + k)] < thr)
+    if (A.cs[12 * (size_t)(a + k)] < thr) {
       mx = max(mx, (unsigned long long)__double_as_longlong(A.densg[g]));
-    else
+      A.pos_of[g] = -1;  // the edge list skips it
+    } else {
       A.GL2[a + A.cnt[a + k] + (i - A.cstart[a + k])] = g;
+    }
   }
   if (mx) atomicMax(&T.pruned_max_bits, mx);
   __syncthreads();
@@ -1410,9 +1566,15 @@ __device__ void follow_phases(const TreeArgs& A, SharedTask& T, int32_t* s_big, 
     if (code == kPhUnion) {
       if (tid == 0) { T.nbig = 0; T.next_event = DBL_MAX; }
       __syncthreads();
-      union_short_rows<NT>(A, a, b, poff, rhot, par, s_big, &T.nbig, &T.next_event, gt, gs);
-      __syncthreads();
-      union_long_rows<NT>(A, a, b, poff, par, s_big, T.nbig);
+      const int32_t ne = LT->nedges;
+      if (ne < 0) {
+        union_short_rows<NT>(A, a, b, poff, rhot, par, s_big, &T.nbig, &T.next_event, gt, gs);
+        __syncthreads();
+        union_long_rows<NT>(A, a, b, poff, par, s_big, T.nbig);
+      } else {
+        union_edges<NT>(A, a, b, ne, poff, rhot, par, &T.next_event, gt, gs);
+        __syncthreads();
+      }
       if (tid == 0) LT->ev_part[rank] = T.next_event;
     } else if (code == kPhFind) {
       find_roots(A, a, b, poff, rhot, par, gt, gs);
@@ -1481,6 +1643,7 @@ __global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : 4) tree_wave_kernel(TreeA
     T.has_cont = 0;
     T.npruned = 0;
     T.pruned_max_bits = 0ull;
+    T.nedges = -1;
   }
   __syncthreads();
   while (true) {
@@ -1755,7 +1918,7 @@ __global__ void pair_sums_kernel(const TreeArgs A, const unsigned long long* __r
   const int32_t N = (int32_t)(keys[p] >> 32), g = (int32_t)(keys[p] & 0xffffffffu);
   if (A.goff[g + 1] - A.goff[g] > kBigGroup) return;
   const int32_t ref = posref[N];
-  group_sums_thread(A, g, A.node[N].rho_saddle, A.x[ref], A.y[ref], A.z[ref], ps + 8 * p);
+  group_sums_thread(A, g, A.node[N].rho_saddle, A.x[ref], A.y[ref], A.z[ref], ps + 8 * p, 1);
 }
 
 // the same for pairs of large groups, a warp per pair
@@ -1770,7 +1933,7 @@ __global__ void __launch_bounds__(256) pair_sums_warp_kernel(const TreeArgs A,
     const int32_t N = (int32_t)(keys[p] >> 32), g = (int32_t)(keys[p] & 0xffffffffu);
     if (A.goff[g + 1] - A.goff[g] <= kBigGroup) continue;
     const int32_t ref = posref[N];
-    group_sums_warp(A, g, A.node[N].rho_saddle, A.x[ref], A.y[ref], A.z[ref], ps + 8 * p, st[wib], lane);
+    group_sums_warp(A, g, A.node[N].rho_saddle, A.x[ref], A.y[ref], A.z[ref], ps + 8 * p, 1, st[wib], lane);
   }
 }
 
@@ -2111,7 +2274,7 @@ int stage_nodes(Engine& E) {
   const size_t bytes_i = G * 4;
   // every sub-array starts on a 256-byte boundary: size the buffer with the rounding
   auto r256 = [](size_t b) { return (b + 255) & ~size_t(255); };
-  const size_t need = r256(bytes_i) * 12 + r256(bytes_i * kClusterCtas) * 2 + r256(G * 8 * 8) + r256(G * 12 * 8) +
+  const size_t need = r256(bytes_i) * 13 + r256(G * sizeof(EdgeRec)) + r256(bytes_i * kClusterCtas) * 2 + r256(G * 8 * 8) + r256(G * 12 * 8) +
                       r256((size_t)(nnodesmax + 1) * sizeof(Task)) * 4 + r256((size_t)(nnodesmax + 1) * 4) * 4;
   AHOP_CUDA_TRY(E.d_tree_scratch.ensure(need));
   char* p = static_cast<char*>(E.d_tree_scratch.p);
@@ -2129,6 +2292,8 @@ int stage_nodes(Engine& E) {
   A.deepnode = reinterpret_cast<int32_t*>(take(bytes_i));
   A.gcur = reinterpret_cast<int32_t*>(take(bytes_i));
   A.ecur = reinterpret_cast<int32_t*>(take(bytes_i));
+  A.ecnt = reinterpret_cast<int32_t*>(take(bytes_i));
+  A.elist = reinterpret_cast<EdgeRec*>(take(G * sizeof(EdgeRec)));
   A.rcnt = reinterpret_cast<int32_t*>(take(bytes_i * kClusterCtas));
   A.rrun = reinterpret_cast<int32_t*>(take(bytes_i * kClusterCtas));
   A.gs = reinterpret_cast<double*>(take(G * 8 * 8));
