@@ -297,7 +297,7 @@ typedef struct {
   double pairs;                                    /* sum over halos of n(n-1)/2 */
   int32_t items, kernel_launches;
   float tune_ms;          /* host wall time of the tile autotuner in this call (0 when it did not run) */
-  int32_t graph_replays;  /* replays of the captured launch graph since its capture (-1: graphs off) */
+  int32_t graph_replays;  /* launches of the captured graph since its capture (0: launched directly, -1: graphs off) */
 } AhopHaloTimings;
 
 /* Host buffers: off[nhalo+1], pos[n][3], vel[n][3], mass[n], density[n];
@@ -324,9 +324,10 @@ int ahop_halo_get_timings(AhopHaloTimings* t);
 #define AHOP_HALO_BUCKETS 5
 int ahop_halo_get_tiles(int32_t* rows, float* ms);
 int ahop_halo_set_tiles(const int32_t* rows);
-/* The launch sequence of ahop_halo_props(_device) is captured once as a CUDA
- * graph and replayed while the call's device pointers, halo count and work
- * list sizes stay the same (on = 1, the default); on = 0 launches directly. */
+/* The launch sequence of ahop_halo_props(_device) is captured as a CUDA graph
+ * by the second call in a row with the same device pointers, halo count and
+ * work list sizes, and replayed while they stay the same (on = 1, the
+ * default); on = 0 always launches directly. */
 int ahop_halo_set_graph(int32_t on);
 /* Allocation-free variant of ahop_halo_props_device (no counterpart in the
  * reference).  For callers that cannot call cudaMalloc -- code running while
