@@ -40,7 +40,7 @@ static int ensure_device(Engine& E) {
   }
   if (!E.events_ready) {
     for (auto& e : E.ev) AHOP_CUDA_TRY(cudaEventCreate(&e));
-    AHOP_CUDA_TRY(cudaMallocHost(&E.h_scalars, 64));
+    AHOP_CUDA_TRY(cudaMallocHost(&E.h_scalars, 8 * Engine::kHostScalars));
     E.events_ready = true;
   }
   return AHOP_OK;
@@ -100,13 +100,20 @@ static int run_pipeline(Engine& E, const double* d_pos, const double* d_mass, in
     AHOP_CUDA_TRY(cudaEventRecord(E.ev_copied, E.stream_copy));
   }
   AHOP_CUDA_TRY(cudaEventRecord(E.ev[3], st));
-  if (last_stage < 3) return AHOP_OK;
+  if (last_stage < 3) {
+    AHOP_CUDA_TRY(cudaStreamSynchronize(st));
+    return knn_failed(E) ? AHOP_ELIMIT : AHOP_OK;
+  }
   if ((rc = stage_hop_groups(E))) return rc;
   AHOP_CUDA_TRY(cudaEventRecord(E.ev[4], st));
   if (last_stage < 4) return AHOP_OK;
   if ((rc = stage_saddles(E))) return rc;
   AHOP_CUDA_TRY(cudaEventRecord(E.ev[5], st));
-  if (last_stage < 5) return AHOP_OK;
+  if (last_stage < 5) {
+    AHOP_CUDA_TRY(cudaStreamSynchronize(st));
+    saddles_counted(E);
+    return AHOP_OK;
+  }
   if ((rc = stage_nodes(E))) return rc;
   AHOP_CUDA_TRY(cudaEventRecord(E.ev[6], st));
   AHOP_CUDA_TRY(cudaEventRecord(E.ev[7], st));

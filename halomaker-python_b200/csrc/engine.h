@@ -11,17 +11,28 @@
 
 namespace ahop {
 
-// Growable device buffer; never shrinks until close().
+// Growable device buffer; never shrinks until close().  A buffer that has to
+// grow takes an eighth more (when there is room): its size follows counts that
+// differ a little from one snapshot to the next, and each growth is a
+// cudaFree and a cudaMalloc (16.7M particles: up to 20 ms of a call).
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
   cudaError_t ensure(size_t need) {
     if (need <= bytes) return cudaSuccess;
+    size_t want = p ? need + need / 8 : need;
     if (p) cudaFree(p);
     p = nullptr;
     bytes = 0;
-    cudaError_t e = cudaMalloc(&p, need ? need : 16);
-    if (e == cudaSuccess) bytes = need ? need : 16;
+    if (!want) want = 16;
+    cudaError_t e = cudaMalloc(&p, want);
+    if (e != cudaSuccess && want > need && need) {
+      cudaGetLastError();
+      want = need;
+      e = cudaMalloc(&p, want);
+    }
+    if (e == cudaSuccess) bytes = want;
+    else p = nullptr;
     return e;
   }
   void release() {
@@ -76,6 +87,8 @@ constexpr int kLeaf = 32;         // particles per leaf bucket
 constexpr int kFan = 32;          // children per internal node
 constexpr int kMaxLevels = 8;
 constexpr int kMaxProfiledWaves = 64;
+// parts of the small flag block d_flags (512 bytes, cleared before the kNN)
+constexpr int kFlagHop = 320;
 constexpr int kProfRow = 32;  // int64 entries per structure-tree task-profile row
 
 struct Engine {
@@ -167,8 +180,9 @@ struct Engine {
   HostBuf h_liste, h_itab, h_dens, h_rtab;
   int64_t h_n = 0, h_nused = 0;
 
-  // small pinned host scalars
+  // small pinned host scalars; the last is the kNN's error flag
   int64_t* h_scalars = nullptr;
+  static constexpr int kHostScalars = 16;
 };
 
 Engine& engine();
@@ -177,8 +191,10 @@ void set_error(const std::string& s);
 // Stage entry points (return AHOP_* codes).
 int stage_sort_and_tree(Engine& E, const double* d_pos_aos, const double* d_mass);
 int stage_knn_density(Engine& E);
+bool knn_failed(Engine& E);  // after a synchronisation of the stream: the kNN kernels' error, with set_error
 int stage_hop_groups(Engine& E);
 int stage_saddles(Engine& E);
+void saddles_counted(Engine& E);  // after a synchronisation of the stream: sets nconn
 int stage_nodes(Engine& E);
 void release_adjoint_memory();  // workspaces of the gradients (adjoint.cu)
 void release_reader_memory();   // staging of the part-file reader (ramses.cu)

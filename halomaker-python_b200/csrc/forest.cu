@@ -53,9 +53,10 @@ __device__ __forceinline__ unsigned long long edge_key(int32_t g, int32_t h) {
   return ((unsigned long long)(unsigned)lo << 32) | (unsigned)hi;
 }
 
-__global__ void forest_init_kernel(ForestArgs F) {
-  const int32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g > F.ng) return;
+// One Boruvka round is the steps best, key, pick, hook, jump, relabel and
+// reset over groups or component roots g; the kernels below run them over the
+// grid or, for few groups, in one block.
+__device__ void forest_init(const ForestArgs& F, int32_t g) {
   F.comp[g] = g;
   F.cur[g] = 0;
   F.gbest[g] = -1;
@@ -65,20 +66,19 @@ __global__ void forest_init_kernel(ForestArgs F) {
   if (g < 3) F.ctr[g] = 0;
 }
 
-// a warp per group: heaviest entry of the row leading to another component
-__global__ void forest_best_kernel(ForestArgs F) {
-  const int32_t g = (int32_t)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) + 1;
-  const int lane = threadIdx.x & 31;
-  if (g > F.ng) return;
+// W lanes of a warp per group (lane of them, sm their mask): heaviest entry of
+// the row leading to another component
+template <int W>
+__device__ void forest_best(const ForestArgs& F, int32_t g, int lane, unsigned sm) {
   const int32_t c = F.comp[g];
   const int32_t base = F.soff[g - 1], e1 = F.soff[g];
   int32_t first = -1;
-  for (int32_t e = base + F.cur[g]; e < e1; e += 32) {
+  for (int32_t e = base + F.cur[g]; e < e1; e += W) {
     const int32_t ee = e + lane;
     const bool cross = ee < e1 && F.comp[F.sisad[ee]] != c;
-    const unsigned m = __ballot_sync(0xffffffffu, cross);
+    const unsigned m = __ballot_sync(sm, cross) & sm;
     if (m) {
-      first = e + __ffs(m) - 1;
+      first = e + __ffs(m) - __ffs(sm);
       break;
     }
   }
@@ -91,7 +91,7 @@ __global__ void forest_best_kernel(ForestArgs F) {
   const double w = F.srho[first];
   unsigned long long bkey = ~0ULL;
   int32_t be = -1;
-  for (int32_t e = first; e < e1; e += 32) {
+  for (int32_t e = first; e < e1; e += W) {
     const int32_t ee = e + lane;
     const bool in = ee < e1 && F.srho[ee] == w;
     if (in) {
@@ -101,12 +101,12 @@ __global__ void forest_best_kernel(ForestArgs F) {
         if (k < bkey) { bkey = k; be = ee; }
       }
     }
-    if (!__all_sync(0xffffffffu, in)) break;  // past the run of equal saddles
+    if (!__all_sync(sm, in)) break;  // past the run of equal saddles
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long ok = __shfl_xor_sync(0xffffffffu, bkey, o);
-    const int32_t oe = __shfl_xor_sync(0xffffffffu, be, o);
+  for (int o = W / 2; o > 0; o >>= 1) {
+    const unsigned long long ok = __shfl_xor_sync(sm, bkey, o);
+    const int32_t oe = __shfl_xor_sync(sm, be, o);
     if (ok < bkey) { bkey = ok; be = oe; }
   }
   if (lane == 0) {
@@ -115,9 +115,7 @@ __global__ void forest_best_kernel(ForestArgs F) {
   }
 }
 
-__global__ void forest_key_kernel(ForestArgs F) {
-  const int32_t g = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  if (g > F.ng) return;
+__device__ void forest_key(const ForestArgs& F, int32_t g) {
   const int32_t be = F.gbest[g];
   if (be < 0) return;
   const int32_t c = F.comp[g];
@@ -125,9 +123,7 @@ __global__ void forest_key_kernel(ForestArgs F) {
   atomicMin(&F.bk[c], edge_key(g, F.sisad[be]));
 }
 
-__global__ void forest_pick_kernel(ForestArgs F) {
-  const int32_t g = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  if (g > F.ng) return;
+__device__ void forest_pick(const ForestArgs& F, int32_t g) {
   const int32_t be = F.gbest[g];
   if (be < 0) return;
   const int32_t c = F.comp[g], h = F.sisad[be];
@@ -135,9 +131,8 @@ __global__ void forest_pick_kernel(ForestArgs F) {
     F.bto[c] = F.comp[h];  // the edge's key is unique, so one group per component gets here
 }
 
-__global__ void forest_hook_kernel(ForestArgs F) {
-  const int32_t c = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  if (c > F.ng || F.comp[c] != c) return;
+__device__ void forest_hook(const ForestArgs& F, int32_t c) {
+  if (F.comp[c] != c) return;
   if (F.bw[c] == 0ULL) {
     F.parent[c] = c;
     return;
@@ -159,9 +154,8 @@ __global__ void forest_hook_kernel(ForestArgs F) {
 
 // pointer jumping over the component roots (bounded per launch; the host
 // relaunches while some chain is not finished)
-__global__ void forest_jump_kernel(ForestArgs F) {
-  const int32_t c = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  if (c > F.ng || F.comp[c] != c) return;
+__device__ void forest_jump(const ForestArgs& F, int32_t c) {
+  if (F.comp[c] != c) return;
   for (int it = 0; it < 32; ++it) {
     const int32_t p = F.parent[c];
     const int32_t pp = F.parent[p];
@@ -171,18 +165,82 @@ __global__ void forest_jump_kernel(ForestArgs F) {
   F.ctr[2] = 1;
 }
 
-__global__ void forest_relabel_kernel(ForestArgs F) {
-  const int32_t g = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  if (g > F.ng) return;
+__device__ void forest_relabel(const ForestArgs& F, int32_t g) {
   F.comp[g] = F.parent[F.comp[g]];
 }
 
-__global__ void forest_reset_kernel(ForestArgs F) {
-  const int32_t g = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  if (g > F.ng) return;
+__device__ void forest_reset(const ForestArgs& F, int32_t g) {
   F.bw[g] = 0ULL;
   F.bk[g] = ~0ULL;
   if (g == 1) { F.ctr[1] = 0; F.ctr[2] = 0; }
+}
+
+// the steps over the grid: a thread per group (or root), a warp for `best`
+#define AHOP_FOREST_KERNEL(step)                                        \
+  __global__ void forest_##step##_kernel(ForestArgs F) {                \
+    const int32_t g = blockIdx.x * blockDim.x + threadIdx.x + 1;        \
+    if (g <= F.ng) forest_##step(F, g);                                 \
+  }
+AHOP_FOREST_KERNEL(key)
+AHOP_FOREST_KERNEL(pick)
+AHOP_FOREST_KERNEL(hook)
+AHOP_FOREST_KERNEL(jump)
+AHOP_FOREST_KERNEL(relabel)
+AHOP_FOREST_KERNEL(reset)
+#undef AHOP_FOREST_KERNEL
+__global__ void forest_init_kernel(ForestArgs F) {
+  const int32_t g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g <= F.ng) forest_init(F, g);
+}
+__global__ void forest_best_kernel(ForestArgs F) {
+  const int32_t g = (int32_t)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) + 1;
+  if (g <= F.ng) forest_best<32>(F, g, threadIdx.x & 31, 0xffffffffu);
+}
+
+// The whole forest in one block.  The grid's rounds need a launch per step and
+// the host's answer twice per round, about 70 us; up to kForestBlock groups one
+// block's rounds are shorter (70,001 particles: preparation 0.37 -> 0.26 ms,
+// 262,144: 0.46 -> 0.32, with the other savings of that stage).  ctr[3]: rounds done, -1 if a
+// limit was hit.
+constexpr int32_t kForestBlock = 2048;
+constexpr int kForestThreads = 1024, kForestLanes = 8;  // rows of few groups are short
+__global__ void __launch_bounds__(kForestThreads) forest_block_kernel(ForestArgs F) {
+  const int32_t tid = threadIdx.x;
+  for (int32_t g = tid; g <= F.ng; g += kForestThreads) forest_init(F, g);
+  __syncthreads();
+  int round = 0;
+  for (;; ++round) {
+    if (round > 40) { round = -1; break; }
+    for (int32_t g = tid / kForestLanes + 1; g <= F.ng; g += kForestThreads / kForestLanes)
+      forest_best<kForestLanes>(F, g, tid & (kForestLanes - 1),
+                                ((1u << kForestLanes) - 1) << (tid & 31 & ~(kForestLanes - 1)));
+    __syncwarp();
+    __syncthreads();
+    for (int32_t g = tid + 1; g <= F.ng; g += kForestThreads) forest_key(F, g);
+    __syncthreads();
+    for (int32_t g = tid + 1; g <= F.ng; g += kForestThreads) forest_pick(F, g);
+    __syncthreads();
+    for (int32_t g = tid + 1; g <= F.ng; g += kForestThreads) forest_hook(F, g);
+    __syncthreads();
+    const bool hooked = atomicAdd(&F.ctr[1], 0) != 0;
+    __syncthreads();
+    if (!hooked) break;
+    bool more = true;
+    for (int pass = 0; more && pass <= 64; ++pass) {
+      if (tid == 0) F.ctr[2] = 0;
+      __syncthreads();
+      for (int32_t g = tid + 1; g <= F.ng; g += kForestThreads) forest_jump(F, g);
+      __syncthreads();
+      more = atomicAdd(&F.ctr[2], 0) != 0;
+      __syncthreads();
+    }
+    if (more) { round = -1; break; }
+    for (int32_t g = tid + 1; g <= F.ng; g += kForestThreads) forest_relabel(F, g);
+    __syncthreads();
+    for (int32_t g = tid + 1; g <= F.ng; g += kForestThreads) forest_reset(F, g);
+    __syncthreads();
+  }
+  if (tid == 0) F.ctr[3] = round;
 }
 
 // forest CSR: per-row counts, then both directions of every edge
@@ -239,36 +297,46 @@ int build_saddle_forest(Engine& E) {
   int32_t* h = reinterpret_cast<int32_t*>(E.h_scalars);
   const unsigned gb = (unsigned)((G + T - 1) / T);
   const unsigned wb = (unsigned)(((int64_t)ng * 32 + T - 1) / T);
-  E.launches++;
-  forest_init_kernel<<<gb, T, 0, st>>>(F);
-  AHOP_CUDA_TRY(cudaGetLastError());
-  // every round at least halves the number of components that still have an
-  // outgoing edge, so 40 rounds cover any int32 group count
   int round = 0;
-  for (;; ++round) {
-    if (round > 40) { set_error("saddle forest: too many rounds"); return AHOP_ELIMIT; }
-    E.launches += 4;
-    forest_best_kernel<<<wb, T, 0, st>>>(F);
-    forest_key_kernel<<<gb, T, 0, st>>>(F);
-    forest_pick_kernel<<<gb, T, 0, st>>>(F);
-    forest_hook_kernel<<<gb, T, 0, st>>>(F);
+  if (ng <= kForestBlock) {
+    E.launches++;
+    forest_block_kernel<<<1, kForestThreads, 0, st>>>(F);
     AHOP_CUDA_TRY(cudaGetLastError());
-    AHOP_CUDA_TRY(cudaMemcpyAsync(h, F.ctr, 8, cudaMemcpyDeviceToHost, st));
+    AHOP_CUDA_TRY(cudaMemcpyAsync(h, F.ctr, 16, cudaMemcpyDeviceToHost, st));
     AHOP_CUDA_TRY(cudaStreamSynchronize(st));
-    if (h[1] == 0) break;
-    for (int pass = 0;; ++pass) {
-      if (pass > 64) { set_error("saddle forest: pointer jumping did not finish"); return AHOP_ELIMIT; }
-      AHOP_CUDA_TRY(cudaMemsetAsync(F.ctr + 2, 0, 4, st));
-      E.launches++;
-      forest_jump_kernel<<<gb, T, 0, st>>>(F);
-      AHOP_CUDA_TRY(cudaMemcpyAsync(h + 2, F.ctr + 2, 4, cudaMemcpyDeviceToHost, st));
-      AHOP_CUDA_TRY(cudaStreamSynchronize(st));
-      if (h[2] == 0) break;
-    }
-    E.launches += 2;
-    forest_relabel_kernel<<<gb, T, 0, st>>>(F);
-    forest_reset_kernel<<<gb, T, 0, st>>>(F);
+    round = h[3];
+    if (round < 0) { set_error("saddle forest: too many rounds"); return AHOP_ELIMIT; }
+  } else {
+    E.launches++;
+    forest_init_kernel<<<gb, T, 0, st>>>(F);
     AHOP_CUDA_TRY(cudaGetLastError());
+    // every round at least halves the number of components that still have an
+    // outgoing edge, so 40 rounds cover any int32 group count
+    for (;; ++round) {
+      if (round > 40) { set_error("saddle forest: too many rounds"); return AHOP_ELIMIT; }
+      E.launches += 4;
+      forest_best_kernel<<<wb, T, 0, st>>>(F);
+      forest_key_kernel<<<gb, T, 0, st>>>(F);
+      forest_pick_kernel<<<gb, T, 0, st>>>(F);
+      forest_hook_kernel<<<gb, T, 0, st>>>(F);
+      AHOP_CUDA_TRY(cudaGetLastError());
+      AHOP_CUDA_TRY(cudaMemcpyAsync(h, F.ctr, 8, cudaMemcpyDeviceToHost, st));
+      AHOP_CUDA_TRY(cudaStreamSynchronize(st));
+      if (h[1] == 0) break;
+      for (int pass = 0;; ++pass) {
+        if (pass > 64) { set_error("saddle forest: pointer jumping did not finish"); return AHOP_ELIMIT; }
+        AHOP_CUDA_TRY(cudaMemsetAsync(F.ctr + 2, 0, 4, st));
+        E.launches++;
+        forest_jump_kernel<<<gb, T, 0, st>>>(F);
+        AHOP_CUDA_TRY(cudaMemcpyAsync(h + 2, F.ctr + 2, 4, cudaMemcpyDeviceToHost, st));
+        AHOP_CUDA_TRY(cudaStreamSynchronize(st));
+        if (h[2] == 0) break;
+      }
+      E.launches += 2;
+      forest_relabel_kernel<<<gb, T, 0, st>>>(F);
+      forest_reset_kernel<<<gb, T, 0, st>>>(F);
+      AHOP_CUDA_TRY(cudaGetLastError());
+    }
   }
   E.forest_rounds = round;
   const int32_t nfe = h[0];

@@ -3,8 +3,8 @@
 //
 //  * hop target: the densest of {self} and the first nhop neighbours, equal
 //    densities resolved to the smallest particle index (f90:777-793);
-//  * pointer jumping to the terminal peak instead of the Fortran's serial
-//    chain walk (f90:819-845) -- the terminal peak of a chain is unique;
+//  * all chains followed to the terminal peak at once instead of the Fortran's
+//    serial walk (f90:819-845) -- the terminal peak of a chain is unique;
 //  * peaks numbered 1..ngroups in increasing particle index (f90:797-803);
 //  * members of each group in DEcreasing particle index, the order of the
 //    Fortran linked lists (f90:853-861), stored as a CSR (goff, gmem);
@@ -21,11 +21,14 @@ namespace ahop {
 
 __global__ void hop_kernel(const double* __restrict__ dens, const int32_t* __restrict__ nei, int nstore,
                            int nhop, const int32_t* __restrict__ orig, int64_t n, double rhot,
-                           int32_t* __restrict__ hop) {
+                           int32_t* __restrict__ hop, int32_t* __restrict__ root, int32_t* __restrict__ nactive) {
   int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const double ds = s < n ? dens[s] : 0.0;
+  const bool active = s < n && ds > rhot;
+  const int cnt = __syncthreads_count(active);
+  if (threadIdx.x == 0 && cnt) atomicAdd(nactive, cnt);
   if (s >= n) return;
-  double ds = dens[s];
-  if (!(ds > rhot)) { hop[s] = -1; return; }
+  if (!active) { hop[s] = root[s] = -1; return; }
   int32_t best = (int32_t)s;
   double bd = ds;
   int32_t bo = orig[s];
@@ -35,20 +38,28 @@ __global__ void hop_kernel(const double* __restrict__ dens, const int32_t* __res
     int32_t ot = orig[t];
     if (dt > bd || (dt == bd && ot < bo)) { best = t; bd = dt; bo = ot; }
   }
-  hop[s] = best;
+  hop[s] = root[s] = best;
 }
 
-// One pointer-doubling pass: root[s] <- root[root[s]]; flags a change.
-__global__ void jump_kernel(int32_t* __restrict__ root, int64_t n, int* __restrict__ changed) {
-  int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+// Every particle's terminal peak in one launch: each thread follows its chain
+// to the end.  The threads shorten the chains for each other (root[s] moves
+// from the hop target to the peak; a reader sees either, both on the chain),
+// and chains strictly rise in (density, -index), so every walk ends.  Doubling
+// passes, five or six with the host's answer after each: 5,003 particles 0.12 ms
+// more, 16.7M 0.44 ms more (hop stage 2.40 -> 1.96).
+__global__ void root_kernel(int32_t* __restrict__ root, int64_t n, int32_t* __restrict__ err) {
+  const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (s >= n) return;
   int32_t r = root[s];
   if (r < 0) return;
-  int32_t rr = root[r];
-  if (rr != r) {
-    root[s] = rr;
-    *changed = 1;
+  bool done = false;
+  for (int it = 0; it < (1 << 28); ++it) {
+    const int32_t rr = root[r];
+    if (rr == r) { done = true; break; }
+    r = rr;
   }
+  if (!done) *err = 1;
+  root[s] = r;
 }
 
 __global__ void peak_flag_kernel(const int32_t* __restrict__ hop, const int32_t* __restrict__ orig, int64_t n,
@@ -112,26 +123,15 @@ int stage_hop_groups(Engine& E) {
   int32_t* hop = E.d_hop.as<int32_t>();
   int32_t* root = E.d_root.as<int32_t>();
   E.launches++;
+  // counters of the call's flag block: [0] active particles, [1] a chain that did not end
+  int32_t* d_cnt = reinterpret_cast<int32_t*>(E.d_flags.as<char>() + kFlagHop);
   hop_kernel<<<grid, T, 0, st>>>(E.d_dens.as<double>(), E.d_nei.as<int32_t>(), E.nstore, P.nhop,
-                                 E.d_orig.as<int32_t>(), n, P.rho_threshold, hop);
+                                 E.d_orig.as<int32_t>(), n, P.rho_threshold, hop, root, d_cnt);
   AHOP_CUDA_TRY(cudaGetLastError());
-  AHOP_CUDA_TRY(cudaMemcpyAsync(root, hop, n * 4, cudaMemcpyDeviceToDevice, st));
-  // pointer jumping: chains strictly increase (density, -index), so they end
-  // at a self-pointing peak; doubling converges in ceil(log2(chain)) passes.
-  int* d_changed = reinterpret_cast<int*>(E.d_peakflag.p);  // reuse as flag before peak flags
-  int* h_changed = reinterpret_cast<int*>(E.h_scalars);
-  bool converged = false;
-  for (int it = 0; it < 64; ++it) {
-    AHOP_CUDA_TRY(cudaMemsetAsync(d_changed, 0, 4, st));
-    E.launches++;
-    jump_kernel<<<grid, T, 0, st>>>(root, n, d_changed);
-    AHOP_CUDA_TRY(cudaGetLastError());
-    AHOP_CUDA_TRY(cudaMemcpyAsync(h_changed, d_changed, 4, cudaMemcpyDeviceToHost, st));
-    AHOP_CUDA_TRY(cudaStreamSynchronize(st));
-    E.hop_passes = it + 1;
-    if (*h_changed == 0) { converged = true; break; }
-  }
-  if (!converged) { set_error("hop pointer jumping did not converge in 64 passes"); return AHOP_ELIMIT; }
+  E.launches++;
+  root_kernel<<<grid, T, 0, st>>>(root, n, d_cnt + 1);
+  AHOP_CUDA_TRY(cudaGetLastError());
+  E.hop_passes = 1;
   // peaks numbered in increasing particle index
   int32_t* flag = E.d_peakflag.as<int32_t>();
   E.launches++;
@@ -145,10 +145,15 @@ int stage_hop_groups(Engine& E) {
   AHOP_CUDA_TRY(E.d_cub.ensure(tmp));
   E.cub_calls++;
   AHOP_CUDA_TRY(cub::DeviceScan::ExclusiveSum(E.d_cub.p, tmp, flag, scan, (int)(n + 1), st));
-  int32_t ng = 0;
-  AHOP_CUDA_TRY(cudaMemcpyAsync(&ng, scan + n, 4, cudaMemcpyDeviceToHost, st));
+  int32_t* h = reinterpret_cast<int32_t*>(E.h_scalars);
+  AHOP_CUDA_TRY(cudaMemcpyAsync(h, scan + n, 4, cudaMemcpyDeviceToHost, st));
+  AHOP_CUDA_TRY(cudaMemcpyAsync(h + 1, d_cnt, 8, cudaMemcpyDeviceToHost, st));
   AHOP_CUDA_TRY(cudaStreamSynchronize(st));
+  const int32_t ng = h[0];
+  if (knn_failed(E)) return AHOP_ELIMIT;
+  if (h[2]) { set_error("hop chains did not end"); return AHOP_ELIMIT; }
   E.ngroups = ng;
+  E.nactive = h[1];
   AHOP_CUDA_TRY(E.d_densg.ensure((size_t)(ng + 2) * 8));
   AHOP_CUDA_TRY(E.d_gpeak.ensure((size_t)(ng + 2) * 4));
   AHOP_CUDA_TRY(E.d_goff.ensure((size_t)(ng + 2) * 4));
@@ -189,10 +194,6 @@ int stage_hop_groups(Engine& E) {
   AHOP_CUDA_TRY(cub::DeviceRadixSort::SortPairs(E.d_cub.p, tmp, E.d_key.as<unsigned long long>(),
                                                 E.d_key2.as<unsigned long long>(), E.d_idx2.as<int32_t>(),
                                                 E.d_gmem.as<int32_t>(), (int)n, 0, end_bit, st));
-  int32_t nact = 0;
-  AHOP_CUDA_TRY(cudaMemcpyAsync(&nact, E.d_goff.as<int32_t>() + ng + 1, 4, cudaMemcpyDeviceToHost, st));
-  AHOP_CUDA_TRY(cudaStreamSynchronize(st));
-  E.nactive = nact;
   return AHOP_OK;
 }
 

@@ -150,15 +150,22 @@ int stage_sort_and_tree(Engine& E, const double* d_pos, const double* d_mass) {
   morton_kernel<<<grid, T, 0, st>>>(d_pos, n, P.xlong, P.ylong, P.zlong, E.d_key.as<unsigned long long>(),
                                     E.d_idx.as<int32_t>());
   AHOP_CUDA_TRY(cudaGetLastError());
+  // Key bits that order leaves: per axis eight levels below the mean spacing
+  // (an overdensity of 2^24); the order below that only shapes the leaves'
+  // boxes, and every eight bits left out are a pass over the keys (16.7M
+  // particles: 6 passes instead of 8, sort and boxes 3.37 -> 2.95 ms).
+  int levels = 8;
+  while ((int64_t)1 << (3 * (levels - 8)) < n) ++levels;
+  const int begin_bit = std::max(0, 63 - 3 * levels);
   size_t tmp = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, tmp, E.d_key.as<unsigned long long>(),
                                   E.d_key2.as<unsigned long long>(), E.d_idx.as<int32_t>(),
-                                  E.d_idx2.as<int32_t>(), (int)n, 0, 63, st);
+                                  E.d_idx2.as<int32_t>(), (int)n, begin_bit, 63, st);
   AHOP_CUDA_TRY(E.d_cub.ensure(tmp));
   E.cub_calls++;
   AHOP_CUDA_TRY(cub::DeviceRadixSort::SortPairs(E.d_cub.p, tmp, E.d_key.as<unsigned long long>(),
                                                 E.d_key2.as<unsigned long long>(), E.d_idx.as<int32_t>(),
-                                                E.d_idx2.as<int32_t>(), (int)n, 0, 63, st));
+                                                E.d_idx2.as<int32_t>(), (int)n, begin_bit, 63, st));
   E.launches++;
   if (E.mass_pending) {  // host path: the masses were uploaded on the copy stream
     AHOP_CUDA_TRY(cudaStreamWaitEvent(st, E.ev_mass, 0));
@@ -1319,14 +1326,26 @@ int stage_knn_density(Engine& E) {
     E.launches += 3;
   }
   AHOP_CUDA_TRY(cudaEventRecord(E.ev[10], E.stream));
-  int herr = 0;
-  AHOP_CUDA_TRY(cudaMemcpyAsync(&herr, E.d_flags.p, 4, cudaMemcpyDeviceToHost, E.stream));
-  AHOP_CUDA_TRY(cudaMemcpyAsync(E.knn_stats, E.d_flags.as<char>() + 64, 12 * 8, cudaMemcpyDeviceToHost, E.stream));
-  AHOP_CUDA_TRY(cudaMemcpyAsync(E.knn_phase, E.d_flags.as<char>() + 64 + 24 * 8, 5 * 8, cudaMemcpyDeviceToHost,
+  // the error flag is looked at after the next stage's synchronisation
+  AHOP_CUDA_TRY(cudaMemcpyAsync(E.h_scalars + Engine::kHostScalars - 1, E.d_flags.p, 4, cudaMemcpyDeviceToHost,
                                 E.stream));
-  AHOP_CUDA_TRY(cudaStreamSynchronize(E.stream));
-  if (herr) { set_error("kNN traversal stack overflow"); return AHOP_ELIMIT; }
+  if (prof) {
+    AHOP_CUDA_TRY(cudaMemcpyAsync(E.knn_stats, E.d_flags.as<char>() + 64, 12 * 8, cudaMemcpyDeviceToHost, E.stream));
+    AHOP_CUDA_TRY(cudaMemcpyAsync(E.knn_phase, E.d_flags.as<char>() + 64 + 24 * 8, 5 * 8, cudaMemcpyDeviceToHost,
+                                  E.stream));
+    AHOP_CUDA_TRY(cudaStreamSynchronize(E.stream));
+  } else {
+    std::memset(E.knn_stats, 0, sizeof E.knn_stats);
+    std::memset(E.knn_phase, 0, sizeof E.knn_phase);
+  }
   return AHOP_OK;
+}
+
+bool knn_failed(Engine& E) {
+  int32_t e;
+  std::memcpy(&e, E.h_scalars + Engine::kHostScalars - 1, 4);
+  if (e) set_error("kNN traversal stack overflow");
+  return e != 0;
 }
 
 }  // namespace ahop

@@ -57,6 +57,8 @@ __host__ __device__ constexpr int ipt_for(int nt) { return nt >= 1024 ? 2 : kIPT
 // (a 1024-thread launch sizes its array to its largest task, up to this)
 __host__ __device__ constexpr int par_cap(int nt) { return nt >= 1024 ? 32768 : 1024; }
 constexpr int kBigGroup = 96;   // groups larger than this are summed by a warp
+constexpr int kPairWarp = 16;   // the same for the node sums: a thread's members are a chain of loads (262,144
+                                // particles, both kernels: 96: 0.30 ms, 16: 0.12)
 constexpr int kRowWarp = 8;     // saddle-row prefixes longer than this are linked by a warp
 constexpr int kMaxBigRows = 512;
 constexpr long long kMaxTaskLevels = 4000000LL;  // cap on one task's threshold levels (error, never a hang)
@@ -349,7 +351,7 @@ __device__ __forceinline__ void lead_phase(SharedTask& T, int32_t code, bool loc
 // its groups: a forest); later ones come from the list.
 __device__ __forceinline__ void list_edge(const TreeArgs& A, int32_t a, int32_t b, int32_t u, int32_t v, double w) {
   const int32_t s = atomicAdd(&A.ecnt[a], 1);
-  if (s >= b - a) { set_err(A, 19, u); return; }
+  if (s >= b - a) { set_err(A, 21, u); return; }
   EdgeRec r;
   r.u = u; r.v = v; r.w = w;
   A.elist[a + s] = r;
@@ -1169,27 +1171,32 @@ __device__ void group_sums_warp(const TreeArgs& A, int32_t g, double rhot, doubl
   const int32_t q0 = A.goff[g], q1 = A.goff[g + 1];
   int32_t imass = 0;
   double acc = 0.0;  // lane c < 6 carries sum c: truemass, posg(3), rsquare, densmoy
-  for (int32_t base = q0; base < q1; base += 32) {
-    const int32_t q = base + lane;
-    bool ok = false;
-    double t[6];
+  // the next chunk's members are loaded while this chunk's terms are added
+  double nd = -DBL_MAX, nm = 0, nx = 0, ny = 0, nz = 0;
+  auto fetch = [&](int32_t q) {
+    nd = -DBL_MAX;
     if (q < q1) {
       const int32_t s = A.gmem[q];
-      const double d = A.dens[s];
-      if (d > rhot) {
-        ok = true;
-        const double xm = A.m[s];
-        const double ux = xadd(wrapd(xsub(A.x[s], rx), A.Lx, A.hx), rx);
-        const double uy = xadd(wrapd(xsub(A.y[s], ry), A.Ly, A.hy), ry);
-        const double uz = xadd(wrapd(xsub(A.z[s], rz), A.Lz, A.hz), rz);
-        t[0] = xm;
-        t[1] = xmul(ux, xm);
-        t[2] = xmul(uy, xm);
-        t[3] = xmul(uz, xm);
-        t[4] = xmul(xm, xadd(xadd(xmul(ux, ux), xmul(uy, uy)), xmul(uz, uz)));
-        t[5] = d;
-      }
+      nd = A.dens[s]; nm = A.m[s]; nx = A.x[s]; ny = A.y[s]; nz = A.z[s];
     }
+  };
+  fetch(q0 + lane);
+  for (int32_t base = q0; base < q1; base += 32) {
+    const double d = nd, xm = nm, x = nx, y = ny, z = nz;
+    const bool ok = d > rhot;
+    double t[6];
+    if (ok) {
+      const double ux = xadd(wrapd(xsub(x, rx), A.Lx, A.hx), rx);
+      const double uy = xadd(wrapd(xsub(y, ry), A.Ly, A.hy), ry);
+      const double uz = xadd(wrapd(xsub(z, rz), A.Lz, A.hz), rz);
+      t[0] = xm;
+      t[1] = xmul(ux, xm);
+      t[2] = xmul(uy, xm);
+      t[3] = xmul(uz, xm);
+      t[4] = xmul(xm, xadd(xadd(xmul(ux, ux), xmul(uy, uy)), xmul(uz, uz)));
+      t[5] = d;
+    }
+    if (base + 32 < q1) fetch(base + 32 + lane);
     const unsigned m = __ballot_sync(0xffffffffu, ok);
     const int cnt = __popc(m);
     if (ok) {
@@ -1862,29 +1869,30 @@ __global__ void pair_count_kernel(const TreeArgs A, int32_t nn, int32_t* cnt) {
   cnt[g - 1] = d;
 }
 
-__global__ void pair_emit_kernel(const TreeArgs A, const int32_t* __restrict__ off,
+// pair keys: node above gb bits of the group
+__global__ void pair_emit_kernel(const TreeArgs A, const int32_t* __restrict__ off, int gb,
                                  unsigned long long* __restrict__ keys) {
   const int32_t g = blockIdx.x * blockDim.x + threadIdx.x + 1;
   if (g > A.ngroups) return;
   int32_t p = off[g - 1];
   const int32_t p1 = off[g];
   for (int32_t N = A.deepnode[g]; N > 0 && p < p1; N = A.node[N].mother)
-    keys[p++] = ((unsigned long long)N << 32) | (unsigned)g;
+    keys[p++] = ((unsigned long long)N << gb) | (unsigned)g;
 }
 
 // pair range [nstart[N], nend[N]) of every node in the sorted pair keys
-__global__ void node_range_kernel(const unsigned long long* __restrict__ keys, int64_t np, int32_t* nstart,
+__global__ void node_range_kernel(const unsigned long long* __restrict__ keys, int64_t np, int gb, int32_t* nstart,
                                   int32_t* nend) {
   const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (p >= np) return;
-  const int32_t N = (int32_t)(keys[p] >> 32);
-  if (p == 0 || (int32_t)(keys[p - 1] >> 32) != N) nstart[N] = (int32_t)p;
-  if (p == np - 1 || (int32_t)(keys[p + 1] >> 32) != N) nend[N] = (int32_t)(p + 1);
+  const int32_t N = (int32_t)(keys[p] >> gb);
+  if (p == 0 || (int32_t)(keys[p - 1] >> gb) != N) nstart[N] = (int32_t)p;
+  if (p == np - 1 || (int32_t)(keys[p + 1] >> gb) != N) nend[N] = (int32_t)(p + 1);
 }
 
 // posref of every node (f90:2340-2344): the first member, in list order, of
 // its first group above its threshold; a warp per node
-__global__ void node_posref_kernel(const TreeArgs A, int32_t nn, const unsigned long long* __restrict__ keys,
+__global__ void node_posref_kernel(const TreeArgs A, int32_t nn, int gb, const unsigned long long* __restrict__ keys,
                                    const int32_t* __restrict__ nstart, const int32_t* __restrict__ nend,
                                    int32_t* __restrict__ posref) {
   const int32_t N = (int32_t)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) + 1;
@@ -1894,7 +1902,7 @@ __global__ void node_posref_kernel(const TreeArgs A, int32_t nn, const unsigned 
     if (lane == 0) { set_err(A, 20, N); posref[N] = 0; }
     return;
   }
-  const int32_t g0 = (int32_t)(keys[nstart[N]] & 0xffffffffu);
+  const int32_t g0 = (int32_t)(keys[nstart[N]] & ((1ULL << gb) - 1));
   const double rhot = A.node[N].rho_saddle;
   const int32_t q1 = A.goff[g0 + 1];
   for (int32_t base = A.goff[g0]; base < q1; base += 32) {
@@ -1911,12 +1919,12 @@ __global__ void node_posref_kernel(const TreeArgs A, int32_t nn, const unsigned 
 }
 
 // per (node, group) pair sums, a thread per pair of a small group
-__global__ void pair_sums_kernel(const TreeArgs A, const unsigned long long* __restrict__ keys, int64_t np,
+__global__ void pair_sums_kernel(const TreeArgs A, const unsigned long long* __restrict__ keys, int64_t np, int gb,
                                  const int32_t* __restrict__ posref, double* __restrict__ ps) {
   const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (p >= np) return;
-  const int32_t N = (int32_t)(keys[p] >> 32), g = (int32_t)(keys[p] & 0xffffffffu);
-  if (A.goff[g + 1] - A.goff[g] > kBigGroup) return;
+  const int32_t N = (int32_t)(keys[p] >> gb), g = (int32_t)(keys[p] & ((1ULL << gb) - 1));
+  if (A.goff[g + 1] - A.goff[g] > kPairWarp) return;
   const int32_t ref = posref[N];
   group_sums_thread(A, g, A.node[N].rho_saddle, A.x[ref], A.y[ref], A.z[ref], ps + 8 * p, 1);
 }
@@ -1924,14 +1932,14 @@ __global__ void pair_sums_kernel(const TreeArgs A, const unsigned long long* __r
 // the same for pairs of large groups, a warp per pair
 __global__ void __launch_bounds__(256) pair_sums_warp_kernel(const TreeArgs A,
                                                              const unsigned long long* __restrict__ keys,
-                                                             int64_t np, const int32_t* __restrict__ posref,
+                                                             int64_t np, int gb, const int32_t* __restrict__ posref,
                                                              double* __restrict__ ps) {
   __shared__ double st[8][32 * 6];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int64_t nw = (int64_t)gridDim.x * 8;
   for (int64_t p = (int64_t)blockIdx.x * 8 + wib; p < np; p += nw) {
-    const int32_t N = (int32_t)(keys[p] >> 32), g = (int32_t)(keys[p] & 0xffffffffu);
-    if (A.goff[g + 1] - A.goff[g] <= kBigGroup) continue;
+    const int32_t N = (int32_t)(keys[p] >> gb), g = (int32_t)(keys[p] & ((1ULL << gb) - 1));
+    if (A.goff[g + 1] - A.goff[g] <= kPairWarp) continue;
     const int32_t ref = posref[N];
     group_sums_warp(A, g, A.node[N].rho_saddle, A.x[ref], A.y[ref], A.z[ref], ps + 8 * p, 1, st[wib], lane);
   }
@@ -2070,6 +2078,9 @@ __global__ void member_fix_runs_kernel(const unsigned long long* __restrict__ ke
   }
 }
 
+// members above which a group's running sums take a block
+constexpr int32_t kPrefixBlock = 256;
+
 // running sums per group (one warp per group) in decreasing-density order
 __global__ void prefix_moments_kernel(const int32_t* __restrict__ goff, int32_t ng,
                                       const int32_t* __restrict__ mem_rho_order, const double* __restrict__ rdesc,
@@ -2083,16 +2094,27 @@ __global__ void prefix_moments_kernel(const int32_t* __restrict__ goff, int32_t 
   const int32_t p = gpeak[g];
   const double ax = x[p], ay = y[p], az = z[p];
   double c[6] = {0, 0, 0, 0, 0, 0};
-  for (int32_t base = goff[g]; base < goff[g + 1]; base += 32) {
+  const int32_t q0 = goff[g], q1 = goff[g + 1];
+  if (q1 - q0 > kPrefixBlock) return;  // prefix_moments_block_kernel
+  // the next chunk's members are loaded while this chunk's sums are scanned
+  double nw = 0, nx = 0, ny = 0, nz = 0, nr = 0;
+  auto fetch = [&](int32_t q) {
+    if (q < q1) {
+      const int32_t s = mem_rho_order[q];
+      nw = mm[s]; nx = x[s]; ny = y[s]; nz = z[s]; nr = rdesc[q];
+    }
+  };
+  fetch(q0 + lane);
+  for (int32_t base = q0; base < q1; base += 32) {
     const int32_t q = base + lane;
     double v[6] = {0, 0, 0, 0, 0, 0};
-    if (q < goff[g + 1]) {
-      const int32_t s = mem_rho_order[q];
-      const double w = mm[s];
-      double dx = wrapd(x[s] - ax, Lx, hx), dy = wrapd(y[s] - ay, Ly, hy), dz = wrapd(z[s] - az, Lz, hz);
-      v[0] = rdesc[q]; v[1] = w; v[2] = w * dx; v[3] = w * dy; v[4] = w * dz;
+    if (q < q1) {
+      const double w = nw;
+      double dx = wrapd(nx - ax, Lx, hx), dy = wrapd(ny - ay, Ly, hy), dz = wrapd(nz - az, Lz, hz);
+      v[0] = nr; v[1] = w; v[2] = w * dx; v[3] = w * dy; v[4] = w * dz;
       v[5] = w * (dx * dx + dy * dy + dz * dz);
     }
+    if (base + 32 < q1) fetch(q + 32);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
 #pragma unroll
@@ -2101,12 +2123,66 @@ __global__ void prefix_moments_kernel(const int32_t* __restrict__ goff, int32_t 
         if (lane >= o) v[t] += up;
       }
     }
-    if (q < goff[g + 1]) {
+    if (q < q1) {
 #pragma unroll
       for (int t = 0; t < 6; ++t) pref[6 * (size_t)q + t] = c[t] + v[t];
     }
 #pragma unroll
     for (int t = 0; t < 6; ++t) c[t] += __shfl_sync(0xffffffffu, v[t], 31);
+  }
+}
+
+// The same for groups of more than kPrefixBlock members, a block each, 256
+// members per turn: the warps' scans run side by side, then each adds the totals
+// before it.  (A warp per group walked the largest group 32 members at a time:
+// 0.14 ms of a 262,144-particle call, both kernels now 0.05.)
+__global__ void __launch_bounds__(256) prefix_moments_block_kernel(
+    const int32_t* __restrict__ goff, int32_t ng, const int32_t* __restrict__ mem_rho_order,
+    const double* __restrict__ rdesc, const int32_t* __restrict__ gpeak, const double* __restrict__ x,
+    const double* __restrict__ y, const double* __restrict__ z, const double* __restrict__ mm, double Lx, double Ly,
+    double Lz, double hx, double hy, double hz, double* __restrict__ pref) {
+  __shared__ double s_tot[8][6];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int32_t g = blockIdx.x + 1; g <= ng; g += gridDim.x) {
+    const int32_t q0 = goff[g], q1 = goff[g + 1];
+    if (q1 - q0 <= kPrefixBlock) continue;
+    const int32_t p = gpeak[g];
+    const double ax = x[p], ay = y[p], az = z[p];
+    double c[6] = {0, 0, 0, 0, 0, 0};
+    for (int32_t base = q0; base < q1; base += 256) {
+      const int32_t q = base + threadIdx.x;
+      double v[6] = {0, 0, 0, 0, 0, 0};
+      if (q < q1) {
+        const int32_t s = mem_rho_order[q];
+        const double w = mm[s];
+        const double dx = wrapd(x[s] - ax, Lx, hx), dy = wrapd(y[s] - ay, Ly, hy), dz = wrapd(z[s] - az, Lz, hz);
+        v[0] = rdesc[q]; v[1] = w; v[2] = w * dx; v[3] = w * dy; v[4] = w * dz;
+        v[5] = w * (dx * dx + dy * dy + dz * dz);
+      }
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+        for (int t = 0; t < 6; ++t) {
+          const double up = __shfl_up_sync(0xffffffffu, v[t], o);
+          if (lane >= o) v[t] += up;
+        }
+      }
+      if (lane == 31) {
+#pragma unroll
+        for (int t = 0; t < 6; ++t) s_tot[warp][t] = v[t];
+      }
+      __syncthreads();
+#pragma unroll
+      for (int t = 0; t < 6; ++t) {
+        double before = c[t];
+        for (int k = 0; k < 8; ++k) {
+          if (k < warp) before += s_tot[k][t];
+          c[t] += s_tot[k][t];
+        }
+        if (q < q1) pref[6 * (size_t)q + t] = before + v[t];
+      }
+      __syncthreads();
+    }
   }
 }
 
@@ -2147,6 +2223,47 @@ struct NodeLess {
     return ia < ib;
   }
 };
+
+// Nodes before each node, counted pair by pair: for few nodes the merge sort's
+// one block, a chain of comparisons through memory, took 0.10 ms for 59 nodes
+// and 0.14 for 425 (here 0.03).  Block (i, j) compares 256 nodes with 256.
+constexpr int32_t kRankNodes = 4096;
+__global__ void __launch_bounds__(256) node_rank_kernel(const NodeRec* __restrict__ node, int32_t nn,
+                                                        int32_t* __restrict__ rank) {
+  __shared__ int32_t s_level[256], s_n[256];
+  __shared__ double s_mass[256], s_max[256];  // small nodes often tie up to the member count
+  const int32_t i = blockIdx.x * 256 + threadIdx.x + 1, j0 = blockIdx.y * 256 + 1;
+  const int32_t jn = min(256, nn + 1 - j0);
+  if ((int)threadIdx.x < jn) {
+    const NodeRec& b = node[j0 + threadIdx.x];
+    s_level[threadIdx.x] = b.level;
+    s_mass[threadIdx.x] = b.truemass;
+    s_n[threadIdx.x] = b.mass;
+    s_max[threadIdx.x] = b.densmax;
+  }
+  __syncthreads();
+  if (i > nn) return;
+  const NodeLess less{node};
+  const int32_t level = node[i].level, n = node[i].mass;
+  const double mass = node[i].truemass, dmax = node[i].densmax;
+  int32_t before = 0;
+  for (int32_t t = 0; t < jn; ++t) {
+    if (j0 + t == i) continue;
+    bool b;
+    if (s_level[t] != level) b = s_level[t] < level;
+    else if (s_mass[t] > mass || s_mass[t] < mass) b = s_mass[t] > mass;
+    else if (s_n[t] != n && s_mass[t] == mass) b = s_n[t] > n;
+    else if (s_mass[t] == mass && (s_max[t] > dmax || s_max[t] < dmax)) b = s_max[t] > dmax;
+    else b = less(j0 + t, i) || (!less(i, j0 + t) && j0 + t < i);
+    before += b ? 1 : 0;
+  }
+  if (before) atomicAdd(&rank[i], before);
+}
+
+__global__ void node_place_kernel(const int32_t* __restrict__ rank, int32_t nn, int32_t* __restrict__ new_to_old) {
+  const int32_t i = blockIdx.x * blockDim.x + threadIdx.x + 1;
+  if (i <= nn) new_to_old[min(rank[i], nn - 1)] = i;
+}
 
 __global__ void iota_kernel(int32_t* v, int32_t n, int32_t base) {
   int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2205,7 +2322,6 @@ int stage_nodes(Engine& E) {
   double* rho_idx = E.d_gmem_rho.as<double>();        // densities in particle-index order
   double* rdesc = E.d_gmem_rho.as<double>() + nact;   // sorted decreasing
   int32_t* mem_rho = reinterpret_cast<int32_t*>(E.d_sad_val2.p);
-  bool sorted = false;
   if (nact > 0) {
     // one radix sort of (group, density rounded to float), then exact order
     // inside runs of equal keys (member_rho_keys_kernel)
@@ -2232,12 +2348,31 @@ int stage_nodes(Engine& E) {
     AHOP_CUDA_TRY(cudaMemsetAsync(fl, 0, 4, st));
     member_fix_runs_kernel<<<gm, T, 0, st>>>(k1, nact, mem_rho, rdesc, fl);
     AHOP_CUDA_TRY(cudaGetLastError());
-    int32_t* hf = reinterpret_cast<int32_t*>(E.h_scalars);
-    AHOP_CUDA_TRY(cudaMemcpyAsync(hf, fl, 4, cudaMemcpyDeviceToHost, st));
-    AHOP_CUDA_TRY(cudaStreamSynchronize(st));
-    sorted = hf[0] == 0;
+    // looked at after the forest's synchronisation
+    AHOP_CUDA_TRY(cudaMemcpyAsync(E.h_scalars + 4, fl, 4, cudaMemcpyDeviceToHost, st));
   }
-  if (!sorted && nact > 0) {  // a run of more than kMaxKeyRun equal keys: sort the groups' members exactly
+  auto prefix_moments = [&]() -> int {
+    int64_t threads = (int64_t)ng * 32;
+    E.launches++;
+    prefix_moments_kernel<<<(unsigned)((threads + T - 1) / T), T, 0, st>>>(
+        E.d_goff.as<int32_t>(), ng, mem_rho, rdesc, E.d_gpeak.as<int32_t>(), E.d_x.as<double>(),
+        E.d_y.as<double>(), E.d_z.as<double>(), E.d_m.as<double>(), P.xlong, P.ylong, P.zlong, P.xlongs2,
+        P.ylongs2, P.zlongs2, E.d_gmem_rho_pref.as<double>());
+    E.launches++;
+    prefix_moments_block_kernel<<<(unsigned)std::min(ng, 4736), 256, 0, st>>>(
+        E.d_goff.as<int32_t>(), ng, mem_rho, rdesc, E.d_gpeak.as<int32_t>(), E.d_x.as<double>(),
+        E.d_y.as<double>(), E.d_z.as<double>(), E.d_m.as<double>(), P.xlong, P.ylong, P.zlong, P.xlongs2,
+        P.ylongs2, P.zlongs2, E.d_gmem_rho_pref.as<double>());
+    AHOP_CUDA_TRY(cudaGetLastError());
+    return AHOP_OK;
+  };
+  int rc;
+  if ((rc = prefix_moments())) return rc;
+  // ---- maximum spanning forest of the saddle graph: the colours at every
+  // threshold are its components, so the tree links only its edges
+  if ((rc = build_saddle_forest(E))) return rc;  // synchronises
+  saddles_counted(E);
+  if (nact > 0 && (int32_t)E.h_scalars[4] != 0) {  // a run of more than kMaxKeyRun equal keys: sort the groups' members exactly
     E.launches++;
     gather_member_rho<<<(unsigned)((nact + T - 1) / T), T, 0, st>>>(E.d_gmem.as<int32_t>(), E.d_dens.as<double>(),
                                                                     nact, rho_idx);
@@ -2252,21 +2387,7 @@ int stage_nodes(Engine& E) {
                                                                 E.d_gmem.as<int32_t>(), mem_rho, (int)nact, ng,
                                                                 E.d_goff.as<int32_t>() + 1,
                                                                 E.d_goff.as<int32_t>() + 2, st));
-  }
-  {
-    int64_t threads = (int64_t)ng * 32;
-    E.launches++;
-    prefix_moments_kernel<<<(unsigned)((threads + T - 1) / T), T, 0, st>>>(
-        E.d_goff.as<int32_t>(), ng, mem_rho, rdesc, E.d_gpeak.as<int32_t>(), E.d_x.as<double>(),
-        E.d_y.as<double>(), E.d_z.as<double>(), E.d_m.as<double>(), P.xlong, P.ylong, P.zlong, P.xlongs2,
-        P.ylongs2, P.zlongs2, E.d_gmem_rho_pref.as<double>());
-    AHOP_CUDA_TRY(cudaGetLastError());
-  }
-  // ---- maximum spanning forest of the saddle graph: the colours at every
-  // threshold are its components, so the tree links only its edges
-  {
-    const int rc = build_saddle_forest(E);
-    if (rc) return rc;
+    if ((rc = prefix_moments())) return rc;
   }
   AHOP_CUDA_TRY(cudaEventRecord(E.ev[11], st));
   // ---- tree scratch
@@ -2610,33 +2731,35 @@ int stage_nodes(Engine& E) {
       int32_t* nstart = E.d_node_aux.as<int32_t>();
       int32_t* nend = nstart + (nn + 1);
       int32_t* posref = nend + (nn + 1);
+      int gbits = 1;
+      while ((1LL << gbits) <= (int64_t)ng) ++gbits;
       E.launches++;
-      pair_emit_kernel<<<gb1, T, 0, st>>>(A, A.run, k0);
+      pair_emit_kernel<<<gb1, T, 0, st>>>(A, A.run, gbits, k0);
       AHOP_CUDA_TRY(cudaGetLastError());
       int nb = 1;
       while ((1LL << nb) <= (int64_t)nn) ++nb;
       cub::DoubleBuffer<unsigned long long> kb(k0, k1);
       t1 = 0;
-      cub::DeviceRadixSort::SortKeys(nullptr, t1, kb, (int)np, 0, 32 + nb, st);
+      cub::DeviceRadixSort::SortKeys(nullptr, t1, kb, (int)np, 0, gbits + nb, st);
       AHOP_CUDA_TRY(E.d_cub.ensure(t1));
       E.cub_calls++;
-      AHOP_CUDA_TRY(cub::DeviceRadixSort::SortKeys(E.d_cub.p, t1, kb, (int)np, 0, 32 + nb, st));
+      AHOP_CUDA_TRY(cub::DeviceRadixSort::SortKeys(E.d_cub.p, t1, kb, (int)np, 0, gbits + nb, st));
       const unsigned long long* keys = kb.Current();
       AHOP_CUDA_TRY(cudaMemsetAsync(nstart, 0, (size_t)(nn + 1) * 8, st));
       const unsigned pb = (unsigned)((np + T - 1) / T);
       E.launches++;
-      node_range_kernel<<<pb, T, 0, st>>>(keys, np, nstart, nend);
+      node_range_kernel<<<pb, T, 0, st>>>(keys, np, gbits, nstart, nend);
       E.launches++;
-      node_posref_kernel<<<(unsigned)(((int64_t)nn * 32 + T - 1) / T), T, 0, st>>>(A, nn, keys, nstart, nend,
+      node_posref_kernel<<<(unsigned)(((int64_t)nn * 32 + T - 1) / T), T, 0, st>>>(A, nn, gbits, keys, nstart, nend,
                                                                                     posref);
       E.launches++;
-      pair_sums_kernel<<<pb, T, 0, st>>>(A, keys, np, posref, E.d_pair_sums.as<double>());
+      pair_sums_kernel<<<pb, T, 0, st>>>(A, keys, np, gbits, posref, E.d_pair_sums.as<double>());
       int nsm = 148;
       cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, E.device);
       int64_t wblocks = (np + 7) / 8;
       if (wblocks > (int64_t)nsm * 8) wblocks = (int64_t)nsm * 8;
       E.launches++;
-      pair_sums_warp_kernel<<<(unsigned)wblocks, 256, 0, st>>>(A, keys, np, posref, E.d_pair_sums.as<double>());
+      pair_sums_warp_kernel<<<(unsigned)wblocks, 256, 0, st>>>(A, keys, np, gbits, posref, E.d_pair_sums.as<double>());
       E.launches++;
       node_fold_kernel<<<(unsigned)(((int64_t)nn * 32 + T - 1) / T), T, 0, st>>>(A, nn, nstart, nend,
                                                                     E.d_pair_sums.as<double>());
@@ -2660,12 +2783,21 @@ int stage_nodes(Engine& E) {
     E.launches++;
     iota_kernel<<<(unsigned)((nn + T - 1) / T), T, 0, st>>>(new_to_old, nn, 1);
     AHOP_CUDA_TRY(cudaGetLastError());
-    size_t tmp = 0;
-    NodeLess less{A.node};
-    cub::DeviceMergeSort::SortKeys(nullptr, tmp, new_to_old, nn, less, st);
-    AHOP_CUDA_TRY(E.d_cub.ensure(tmp));
-    E.cub_calls++;
-    AHOP_CUDA_TRY(cub::DeviceMergeSort::SortKeys(E.d_cub.p, tmp, new_to_old, nn, less, st));
+    if (nn <= kRankNodes) {
+      AHOP_CUDA_TRY(cudaMemsetAsync(o2n, 0, (size_t)(nn + 1) * 4, st));  // ranks, then the inverse
+      const unsigned nb = (unsigned)((nn + 255) / 256);
+      E.launches += 2;
+      node_rank_kernel<<<dim3(nb, nb), 256, 0, st>>>(A.node, nn, o2n);
+      node_place_kernel<<<nb, 256, 0, st>>>(o2n, nn, new_to_old);
+      AHOP_CUDA_TRY(cudaGetLastError());
+    } else {
+      size_t tmp = 0;
+      NodeLess less{A.node};
+      cub::DeviceMergeSort::SortKeys(nullptr, tmp, new_to_old, nn, less, st);
+      AHOP_CUDA_TRY(E.d_cub.ensure(tmp));
+      E.cub_calls++;
+      AHOP_CUDA_TRY(cub::DeviceMergeSort::SortKeys(E.d_cub.p, tmp, new_to_old, nn, less, st));
+    }
     E.launches++;
     old_to_new_kernel<<<(unsigned)((nn + T - 1) / T), T, 0, st>>>(new_to_old, nn, o2n);
     AHOP_CUDA_TRY(cudaGetLastError());

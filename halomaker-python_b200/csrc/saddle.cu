@@ -15,6 +15,7 @@
 #include <climits>
 #include <string>
 #include <cub/cub.cuh>
+#include <cstring>
 
 #include "engine.h"
 #include "exact.cuh"
@@ -43,7 +44,7 @@ __global__ void link_count_kernel(const int32_t* __restrict__ group, const int32
 
 __global__ void link_emit_kernel(const int32_t* __restrict__ group, const int32_t* __restrict__ nei, int nstore,
                                  int nhop, const double* __restrict__ dens, int64_t n,
-                                 const int32_t* __restrict__ off, unsigned long long* __restrict__ key,
+                                 const int32_t* __restrict__ off, int gb, unsigned long long* __restrict__ key,
                                  double* __restrict__ val) {
   int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (s >= n) return;
@@ -55,7 +56,7 @@ __global__ void link_emit_kernel(const int32_t* __restrict__ group, const int32_
     int32_t t = nei[s * nstore + i];
     int32_t g2 = group[t];
     if (g2 > 0 && g2 != g1) {
-      key[o] = ((unsigned long long)(uint32_t)g1 << 32) | (uint32_t)g2;
+      key[o] = ((unsigned long long)(uint32_t)g1 << gb) | (uint32_t)g2;
       val[o] = fmin(d1, dens[t]);
       ++o;
     }
@@ -68,13 +69,18 @@ struct MaxOp {
 
 // keep mutual pairs; value = min of the two directions
 __global__ void symmetrize_kernel(const unsigned long long* __restrict__ ukey, const double* __restrict__ uval,
-                                  int32_t nu, int32_t* __restrict__ keep, double* __restrict__ sval,
-                                  int32_t* __restrict__ rowcnt) {
+                                  const int32_t* __restrict__ pnu, int32_t nlink, int gb, int32_t* __restrict__ keep,
+                                  double* __restrict__ sval, int32_t* __restrict__ rowcnt) {
   int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nu) return;
+  const int32_t nu = *pnu;
+  if (i >= nu) {
+    if (i <= nlink) keep[i] = 0;
+    return;
+  }
   unsigned long long k = ukey[i];
-  uint32_t g1 = (uint32_t)(k >> 32), g2 = (uint32_t)(k & 0xffffffffu);
-  unsigned long long rk = ((unsigned long long)g2 << 32) | g1;
+  const unsigned long long low = (1ULL << gb) - 1;
+  uint32_t g1 = (uint32_t)(k >> gb), g2 = (uint32_t)(k & low);
+  unsigned long long rk = ((unsigned long long)g2 << gb) | g1;
   int32_t lo = 0, hi = nu - 1, f = -1;
   while (lo <= hi) {
     int32_t mid = (lo + hi) >> 1;
@@ -93,12 +99,13 @@ __global__ void symmetrize_kernel(const unsigned long long* __restrict__ ukey, c
 }
 
 __global__ void compact_kernel(const unsigned long long* __restrict__ ukey, const double* __restrict__ sval,
-                               const int32_t* __restrict__ keep, const int32_t* __restrict__ kpos, int32_t nu,
-                               int32_t* __restrict__ isad, double* __restrict__ rho) {
+                               const int32_t* __restrict__ keep, const int32_t* __restrict__ kpos,
+                               const int32_t* __restrict__ pnu, int gb, int32_t* __restrict__ isad,
+                               double* __restrict__ rho) {
   int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nu || !keep[i]) return;
+  if (i >= *pnu || !keep[i]) return;
   int32_t p = kpos[i];
-  isad[p] = (int32_t)(ukey[i] & 0xffffffffu);
+  isad[p] = (int32_t)(ukey[i] & ((1ULL << gb) - 1));
   rho[p] = sval[i];
 }
 
@@ -127,11 +134,12 @@ int stage_saddles(Engine& E) {
   AHOP_CUDA_TRY(E.d_cub.ensure(tmp));
   E.cub_calls++;
   AHOP_CUDA_TRY(cub::DeviceScan::ExclusiveSum(E.d_cub.p, tmp, cnt, off, (int)(n + 1), st));
-  int32_t nlink = 0;
-  unsigned long long total = 0;
-  AHOP_CUDA_TRY(cudaMemcpyAsync(&nlink, off + n, 4, cudaMemcpyDeviceToHost, st));
-  AHOP_CUDA_TRY(cudaMemcpyAsync(&total, d_total, 8, cudaMemcpyDeviceToHost, st));
+  AHOP_CUDA_TRY(cudaMemcpyAsync(E.h_scalars, off + n, 4, cudaMemcpyDeviceToHost, st));
+  AHOP_CUDA_TRY(cudaMemcpyAsync(E.h_scalars + 1, d_total, 8, cudaMemcpyDeviceToHost, st));
   AHOP_CUDA_TRY(cudaStreamSynchronize(st));
+  int32_t nlink;
+  std::memcpy(&nlink, E.h_scalars, 4);
+  const unsigned long long total = (unsigned long long)E.h_scalars[1];
   if (total > (unsigned long long)INT32_MAX) {
     set_error("saddles: " + std::to_string(total) + " cross-group links exceed 32-bit offsets");
     return AHOP_ELIMIT;
@@ -143,29 +151,30 @@ int stage_saddles(Engine& E) {
   AHOP_CUDA_TRY(E.d_sad_val2.ensure(nl * 8));
   AHOP_CUDA_TRY(E.d_soff.ensure((size_t)(ng + 2) * 4));
   E.nconn = 0;
+  E.h_scalars[Engine::kHostScalars - 2] = 0;
   if (nlink == 0) {
     AHOP_CUDA_TRY(cudaMemsetAsync(E.d_soff.p, 0, (size_t)(ng + 2) * 4, st));
     AHOP_CUDA_TRY(E.d_sisad.ensure(4));
     AHOP_CUDA_TRY(E.d_srho.ensure(8));
     return AHOP_OK;
   }
-  E.launches++;
-  link_emit_kernel<<<grid, T, 0, st>>>(E.d_group.as<int32_t>(), E.d_nei.as<int32_t>(), E.nstore, P.nhop,
-                                       E.d_dens.as<double>(), n, off, E.d_sad_key.as<unsigned long long>(),
-                                       E.d_sad_val.as<double>());
-  AHOP_CUDA_TRY(cudaGetLastError());
-  // sort links by (g1, g2)
   int gb = 1;
   while ((1LL << gb) <= (int64_t)ng + 1) ++gb;
+  E.launches++;
+  link_emit_kernel<<<grid, T, 0, st>>>(E.d_group.as<int32_t>(), E.d_nei.as<int32_t>(), E.nstore, P.nhop,
+                                       E.d_dens.as<double>(), n, off, gb, E.d_sad_key.as<unsigned long long>(),
+                                       E.d_sad_val.as<double>());
+  AHOP_CUDA_TRY(cudaGetLastError());
+  // sort links by (g1, g2), gb bits each
   tmp = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, tmp, E.d_sad_key.as<unsigned long long>(),
                                   E.d_sad_key2.as<unsigned long long>(), E.d_sad_val.as<double>(),
-                                  E.d_sad_val2.as<double>(), nlink, 0, 32 + gb, st);
+                                  E.d_sad_val2.as<double>(), nlink, 0, 2 * gb, st);
   AHOP_CUDA_TRY(E.d_cub.ensure(tmp));
   E.cub_calls++;
   AHOP_CUDA_TRY(cub::DeviceRadixSort::SortPairs(E.d_cub.p, tmp, E.d_sad_key.as<unsigned long long>(),
                                                 E.d_sad_key2.as<unsigned long long>(), E.d_sad_val.as<double>(),
-                                                E.d_sad_val2.as<double>(), nlink, 0, 32 + gb, st));
+                                                E.d_sad_val2.as<double>(), nlink, 0, 2 * gb, st));
   // segmented max over equal keys -> unique directed saddles (ukey in d_sad_key, uval in d_sad_val)
   AHOP_CUDA_TRY(E.d_sad_keep.ensure((size_t)(nlink + 1) * 4));
   AHOP_CUDA_TRY(E.d_sad_kpos.ensure((size_t)(nlink + 2) * 4));
@@ -179,60 +188,58 @@ int stage_saddles(Engine& E) {
   AHOP_CUDA_TRY(cub::DeviceReduce::ReduceByKey(E.d_cub.p, tmp, E.d_sad_key2.as<unsigned long long>(),
                                                E.d_sad_key.as<unsigned long long>(), E.d_sad_val2.as<double>(),
                                                E.d_sad_val.as<double>(), d_nu, MaxOp(), nlink, st));
-  int32_t nu = 0;
-  AHOP_CUDA_TRY(cudaMemcpyAsync(&nu, d_nu, 4, cudaMemcpyDeviceToHost, st));
-  AHOP_CUDA_TRY(cudaStreamSynchronize(st));
-  // mutual pairs and per-row counts
-  int32_t* keep = E.d_sad_keep.as<int32_t>();            // [nu+1]
-  int32_t* kpos = E.d_sad_kpos.as<int32_t>();            // [nu+1]
-  double* sval = E.d_sad_val2.as<double>();               // [nu]
+  // mutual pairs and per-row counts; the counts of unique and of kept entries
+  // (at most nlink) stay on the device: buffers and launches are sized for
+  // nlink, which costs less than asking for them (two round trips of the host)
+  int32_t* keep = E.d_sad_keep.as<int32_t>();            // [nlink+1]
+  int32_t* kpos = E.d_sad_kpos.as<int32_t>();            // [nlink+1]
+  double* sval = E.d_sad_val2.as<double>();               // [nlink]
   AHOP_CUDA_TRY(E.d_sad_cnt.ensure((size_t)(ng + 2) * 4));
   int32_t* rowcnt = E.d_sad_cnt.as<int32_t>();
   AHOP_CUDA_TRY(cudaMemsetAsync(rowcnt, 0, (size_t)(ng + 2) * 4, st));
-  const unsigned gu = (unsigned)((nu + T - 1) / T);
+  const unsigned gu = (unsigned)(((int64_t)nlink + 1 + T - 1) / T);
   E.launches++;
-  symmetrize_kernel<<<gu, T, 0, st>>>(E.d_sad_key.as<unsigned long long>(), E.d_sad_val.as<double>(), nu, keep,
-                                      sval, rowcnt);
+  symmetrize_kernel<<<gu, T, 0, st>>>(E.d_sad_key.as<unsigned long long>(), E.d_sad_val.as<double>(), d_nu, nlink,
+                                      gb, keep, sval, rowcnt);
   AHOP_CUDA_TRY(cudaGetLastError());
-  AHOP_CUDA_TRY(cudaMemsetAsync(keep + nu, 0, 4, st));
   tmp = 0;
-  cub::DeviceScan::ExclusiveSum(nullptr, tmp, keep, kpos, nu + 1, st);
+  cub::DeviceScan::ExclusiveSum(nullptr, tmp, keep, kpos, nlink + 1, st);
   AHOP_CUDA_TRY(E.d_cub.ensure(tmp));
   E.cub_calls++;
-  AHOP_CUDA_TRY(cub::DeviceScan::ExclusiveSum(E.d_cub.p, tmp, keep, kpos, nu + 1, st));
-  int32_t nc = 0;
-  AHOP_CUDA_TRY(cudaMemcpyAsync(&nc, kpos + nu, 4, cudaMemcpyDeviceToHost, st));
-  AHOP_CUDA_TRY(cudaStreamSynchronize(st));
-  E.nconn = nc;
-  const size_t ncs = (size_t)(nc > 0 ? nc : 1);
-  AHOP_CUDA_TRY(E.d_sisad.ensure(ncs * 4));
-  AHOP_CUDA_TRY(E.d_srho.ensure(ncs * 8));
+  AHOP_CUDA_TRY(cub::DeviceScan::ExclusiveSum(E.d_cub.p, tmp, keep, kpos, nlink + 1, st));
+  // read by saddles_counted after the next synchronisation
+  AHOP_CUDA_TRY(cudaMemcpyAsync(E.h_scalars + Engine::kHostScalars - 2, kpos + nlink, 4, cudaMemcpyDeviceToHost, st));
+  AHOP_CUDA_TRY(E.d_sisad.ensure(nl * 4));
+  AHOP_CUDA_TRY(E.d_srho.ensure(nl * 8));
   // row offsets over groups: soff[g-1] .. soff[g] for group g (rowcnt index g)
   tmp = 0;
   cub::DeviceScan::ExclusiveSum(nullptr, tmp, rowcnt + 1, E.d_soff.as<int32_t>(), ng + 1, st);
   AHOP_CUDA_TRY(E.d_cub.ensure(tmp));
   E.cub_calls++;
   AHOP_CUDA_TRY(cub::DeviceScan::ExclusiveSum(E.d_cub.p, tmp, rowcnt + 1, E.d_soff.as<int32_t>(), ng + 1, st));
-  if (nc == 0) return AHOP_OK;
   // compacted (g1, g2) order == row order by g1; scatter then sort each row by decreasing saddle
+  int32_t* isad = reinterpret_cast<int32_t*>(E.d_sad_key2.p);  // the sorted link keys are no longer needed
   E.launches++;
-  compact_kernel<<<gu, T, 0, st>>>(E.d_sad_key.as<unsigned long long>(), sval, keep, kpos, nu,
-                                   E.d_sisad.as<int32_t>(), E.d_sad_val.as<double>());
+  compact_kernel<<<gu, T, 0, st>>>(E.d_sad_key.as<unsigned long long>(), sval, keep, kpos, d_nu, gb, isad,
+                                   E.d_sad_val.as<double>());
   AHOP_CUDA_TRY(cudaGetLastError());
   // segmented sort by value descending within each row (payload: neighbour id)
-  AHOP_CUDA_TRY(E.d_sad_key2.ensure(ncs * 8));
-  int32_t* isad_sorted = reinterpret_cast<int32_t*>(E.d_sad_key2.p);
   tmp = 0;
   cub::DeviceSegmentedSort::StableSortPairsDescending(nullptr, tmp, E.d_sad_val.as<double>(), E.d_srho.as<double>(),
-                                                      E.d_sisad.as<int32_t>(), isad_sorted, nc, ng,
+                                                      isad, E.d_sisad.as<int32_t>(), nlink, ng,
                                                       E.d_soff.as<int32_t>(), E.d_soff.as<int32_t>() + 1, st);
   AHOP_CUDA_TRY(E.d_cub.ensure(tmp));
   E.cub_calls++;
   AHOP_CUDA_TRY(cub::DeviceSegmentedSort::StableSortPairsDescending(
-      E.d_cub.p, tmp, E.d_sad_val.as<double>(), E.d_srho.as<double>(), E.d_sisad.as<int32_t>(), isad_sorted, nc,
-      ng, E.d_soff.as<int32_t>(), E.d_soff.as<int32_t>() + 1, st));
-  AHOP_CUDA_TRY(cudaMemcpyAsync(E.d_sisad.p, isad_sorted, (size_t)nc * 4, cudaMemcpyDeviceToDevice, st));
+      E.d_cub.p, tmp, E.d_sad_val.as<double>(), E.d_srho.as<double>(), isad, E.d_sisad.as<int32_t>(), nlink, ng,
+      E.d_soff.as<int32_t>(), E.d_soff.as<int32_t>() + 1, st));
   return AHOP_OK;
+}
+
+void saddles_counted(Engine& E) {
+  int32_t c;
+  std::memcpy(&c, E.h_scalars + Engine::kHostScalars - 2, 4);
+  E.nconn = c;
 }
 
 }  // namespace ahop
