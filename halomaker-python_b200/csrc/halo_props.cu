@@ -868,13 +868,13 @@ __device__ __forceinline__ float norm_ru(double x, double y, double z) {
   return __double2float_ru(sqrt(x * x + y * y + z * z) * (1.0 + 1e-12));
 }
 
-// Stage partners [j0, j0 + T) (T = 128 R) of one item relative to the origin
+// Stage partners [j0, j0 + T) (T a multiple of 128) of one item relative to the origin
 // o, with the box and radius bound of every group of 32; slots past j1 get the
 // padding (mass 0, far away) and stay out of the bounds.
-template <int R>
-__device__ __forceinline__ void stage_tile32(Tile32& S, const HaloArgs& A, int64_t base, int32_t j0, int32_t j1,
-                                             double cx, double cy, double cz, double ox, double oy, double oz) {
-  constexpr int P = kB32 * R / 2;  // a multiple of 32: a warp is in or out of an iteration as a whole
+__device__ __forceinline__ void stage_tile32(int T, Tile32& S, const HaloArgs& A, int64_t base, int32_t j0,
+                                             int32_t j1, double cx, double cy, double cz, double ox, double oy,
+                                             double oz) {
+  const int P = T / 2;  // a multiple of 32: a warp is in or out of an iteration as a whole
   for (int q = threadIdx.x; q < P; q += kB32) {
     float hx[2], hy[2], hz[2], m[2], lx[2], ly[2], lz[2];
     float blx = FLT_MAX, bly = FLT_MAX, blz = FLT_MAX, bhx = -FLT_MAX, bhy = -FLT_MAX, bhz = -FLT_MAX, bm = 0.f;
@@ -1035,7 +1035,7 @@ __device__ double epot32_item(Tile32& S, double* sh, double* sred, const HaloArg
   // a warp without rows takes the far form: its sums are discarded
   const bool wvalid = whx >= wlx;
   for (int32_t j0 = it.j0; j0 < it.j1; j0 += T) {
-    stage_tile32<R>(S, A, base, j0, it.j1, cx, cy, cz, ox, oy, oz);
+    stage_tile32(T, S, A, base, j0, it.j1, cx, cy, cz, ox, oy, oz);
     __syncthreads();
     const int jend = min(T, it.j1 - j0);
     if (j0 == it.i0 || checked) {
@@ -1155,6 +1155,179 @@ __global__ void __launch_bounds__(kB32, 4) epot32_kernel(HaloArgs A, const PairI
       else if (code == 1) tot = epot32_item<2>(S, sh, sred, A, it, true);
       else tot = epot32_item<1>(S, sh, sred, A, it, true);
     }
+    if (tid == 0) part[w] = tot;
+  }
+}
+
+// 128 rows of an item, one per thread, for lists that split_items has cut: the
+// item has the rows of shape `code` and starts at the multiple of T below it.i0.
+// Everything that a row's result depends on stays the whole item's: its origin,
+// the box of the warp that owns the row there, the groups of partners in order,
+// the per-pair diagonal tile.  So a row's FP32 sum has the same bits as in
+// epot32_item, and only the FP64 fold of the rows is grouped in another way.
+// (A zero separation sends a part, not the whole item, to the per-pair form.)
+// The shape is a run-time value: with a body for each the compiler kept their
+// common loads alive across them and spilled.
+__device__ double epot32_part(int code, Tile32& S, double* sh, double* sred, const HaloArgs& A, const PairItem& it,
+                              bool checked) {
+  constexpr int NW = kB32 / 32;
+  const int R = 1 << code, T = kB32 << code;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int64_t base = A.off[it.h];
+  const int32_t n = (int32_t)(A.off[it.h + 1] - base);
+  const double* cen = A.out + (size_t)kHaloFields * it.h;
+  const double cx = cen[HP_PX], cy = cen[HP_PY], cz = cen[HP_PZ];
+  const int32_t i0 = it.i0 / T * T;  // first row of the item
+  // origin: centre of the box of the item's rows
+  double lo3[3] = {DBL_MAX, DBL_MAX, DBL_MAX}, hi3[3] = {-DBL_MAX, -DBL_MAX, -DBL_MAX};
+#pragma unroll 1
+  for (int r = 0; r < R; ++r) {
+    const int32_t k = i0 + kB32 * r + tid;
+    if (k >= n) break;
+    double rx, ry, rz, mm;
+    member_rel(A, base + k, cx, cy, cz, rx, ry, rz, mm);
+    lo3[0] = fmin(lo3[0], rx); hi3[0] = fmax(hi3[0], rx);
+    lo3[1] = fmin(lo3[1], ry); hi3[1] = fmax(hi3[1], ry);
+    lo3[2] = fmin(lo3[2], rz); hi3[2] = fmax(hi3[2], rz);
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      lo3[k] = fmin(lo3[k], __shfl_xor_sync(0xffffffffu, lo3[k], o));
+      hi3[k] = fmax(hi3[k], __shfl_xor_sync(0xffffffffu, hi3[k], o));
+    }
+    if (lane == 0) { sred[k * NW + wid] = lo3[k]; sred[(3 + k) * NW + wid] = hi3[k]; }
+  }
+  __syncthreads();
+  double o3[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    double l = sred[k * NW], h = sred[(3 + k) * NW];
+    for (int w = 1; w < NW; ++w) { l = fmin(l, sred[k * NW + w]); h = fmax(h, sred[(3 + k) * NW + w]); }
+    o3[k] = 0.5 * (l + h);
+  }
+  const double ox = o3[0], oy = o3[1], oz = o3[2];
+  // box and radius bound of the rows of the item's warp that owns this row, and
+  // the row itself; padding rows are far on the other side from the padding
+  float wlx = FLT_MAX, wly = FLT_MAX, wlz = FLT_MAX, whx = -FLT_MAX, why = -FLT_MAX, whz = -FLT_MAX, wrho = 0.f;
+  float hx = -kFar, hy = -kFar, hz = -kFar, lx = 0.f, ly = 0.f, lz = 0.f;
+  const int32_t row = it.i0 + tid;
+  const int32_t w0 = it.i0 + 32 * wid - (it.i0 + 32 * wid - i0) % (32 * R);
+#pragma unroll 1
+  for (int r = 0; r < R; ++r) {
+    const int32_t k = w0 + 32 * r + lane;
+    if (k >= n) break;
+    double rx, ry, rz, mm;
+    member_rel(A, base + k, cx, cy, cz, rx, ry, rz, mm);
+    const double bx = rx - ox, by = ry - oy, bz = rz - oz;
+    wlx = fminf(wlx, __double2float_rd(bx)); whx = fmaxf(whx, __double2float_ru(bx));
+    wly = fminf(wly, __double2float_rd(by)); why = fmaxf(why, __double2float_ru(by));
+    wlz = fminf(wlz, __double2float_rd(bz)); whz = fmaxf(whz, __double2float_ru(bz));
+    wrho = fmaxf(wrho, norm_ru(bx, by, bz));
+    if (k == row) {
+      split_hilo(bx, hx, lx);
+      split_hilo(by, hy, ly);
+      split_hilo(bz, hz, lz);
+    }
+  }
+  const f2_t HX = f2_pack(hx, hx), HY = f2_pack(hy, hy), HZ = f2_pack(hz, hz);
+  const f2_t LX = f2_pack(lx, lx), LY = f2_pack(ly, ly), LZ = f2_pack(lz, lz);
+  f2_t ks = 0ull, kc = 0ull;
+  float ksd = 0.f, kcd = 0.f;  // per-pair path sums
+  warp_minmax_f(wlx, whx);
+  warp_minmax_f(wly, why);
+  warp_minmax_f(wlz, whz);
+  float dummy = 0.f;
+  warp_minmax_f(dummy, wrho);
+  const bool wvalid = whx >= wlx;
+  for (int32_t j0 = it.j0; j0 < it.j1; j0 += T) {
+    stage_tile32(T, S, A, base, j0, it.j1, cx, cy, cz, ox, oy, oz);
+    __syncthreads();
+    const int jend = min(T, it.j1 - j0);
+    if (j0 == i0 || checked) {
+      if (row < n)
+        for (int jj = j0 == i0 ? row - i0 + 1 : 0; jj < jend; ++jj) pair_checked(S, jj, hx, hy, hz, lx, ly, lz, ksd, kcd);
+    } else {
+      const int np = ((jend + 2 * kGroup32 - 1) / (2 * kGroup32)) * kGroup32;  // partner pairs, padded
+      const ulonglong2* Sa = reinterpret_cast<const ulonglong2*>(S.a);
+      const ulonglong2* Sb = reinterpret_cast<const ulonglong2*>(S.b);
+      const ulonglong2* Sc = reinterpret_cast<const ulonglong2*>(S.c);
+      const f2_t* Sd = reinterpret_cast<const f2_t*>(S.d);
+      for (int q0 = 0; q0 < np; q0 += kGroup32) {
+        const float4 gl = S.glo[q0 / kGroup32], gh = S.ghi[q0 / kGroup32];
+        const float gx = fmaxf(0.f, fmaxf(gl.x - whx, wlx - gh.x));
+        const float gy = fmaxf(0.f, fmaxf(gl.y - why, wly - gh.y));
+        const float gz = fmaxf(0.f, fmaxf(gl.z - whz, wlz - gh.z));
+        const float dist2 = gx * gx + gy * gy + gz * gz;
+        const float num = wrho + gl.w;
+        const bool far = !wvalid || (dist2 > 0.f && num * num <= kFarK2 * dist2);
+        f2_t acc = 0ull;
+        if (far) {
+#pragma unroll 4
+          for (int g = 0; g < kGroup32; ++g) {
+            const ulonglong2 pa = Sa[q0 + g], pb = Sb[q0 + g];
+            const f2_t dx = f2_sub(pa.x, HX), dy = f2_sub(pa.y, HY), dz = f2_sub(pb.x, HZ);
+            const f2_t r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz)));
+            float u, v;
+            f2_unpack(r2, u, v);
+            acc = f2_fma(pb.y, f2_pack(rsqrt_ftz(u), rsqrt_ftz(v)), acc);
+          }
+        } else {
+#pragma unroll 4
+          for (int g = 0; g < kGroup32; ++g) {
+            const ulonglong2 pa = Sa[q0 + g], pb = Sb[q0 + g], pc = Sc[q0 + g];
+            const f2_t pd = Sd[q0 + g];
+            const f2_t dx = f2_add(f2_sub(pa.x, HX), f2_sub(pc.x, LX));
+            const f2_t dy = f2_add(f2_sub(pa.y, HY), f2_sub(pc.y, LY));
+            const f2_t dz = f2_add(f2_sub(pb.x, HZ), f2_sub(pd, LZ));
+            const f2_t r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz)));
+            float u, v;
+            f2_unpack(r2, u, v);
+            acc = f2_fma(pb.y, f2_pack(rsqrt_ftz(u), rsqrt_ftz(v)), acc);
+          }
+        }
+        const f2_t y = f2_sub(acc, kc);
+        const f2_t s2 = f2_add(ks, y);
+        kc = f2_sub(f2_sub(s2, ks), y);
+        ks = s2;
+      }
+    }
+    __syncthreads();
+  }
+  double mine = 0.0;
+  if (row < n) {
+    float s0, s1, c0, c1;
+    f2_unpack(ks, s0, s1);
+    f2_unpack(kc, c0, c1);
+    const double sum = (((double)s0 - (double)c0) + ((double)s1 - (double)c1)) + ((double)ksd - (double)kcd);
+    double rx, ry, rz, mm;
+    member_rel(A, base + row, cx, cy, cz, rx, ry, rz, mm);
+    mine = mm * sum;
+  }
+  return block_sum<double, kB32>(mine, sh);
+}
+
+// The FP32-compensated pair kernel for a list of parts (split_items).
+__global__ void __launch_bounds__(kB32, 6)
+    epot32_part_kernel(HaloArgs A, const PairItem* __restrict__ items, const int8_t* __restrict__ hshape,
+                       int32_t nitems, int32_t* __restrict__ counter, double* __restrict__ part) {
+  __shared__ Tile32 S;
+  __shared__ double sh[kB32 / 32];
+  __shared__ double sred[6 * (kB32 / 32)];
+  __shared__ int32_t s_item;
+  const int tid = threadIdx.x;
+  for (;;) {
+    if (tid == 0) s_item = atomicAdd(counter, 1);
+    __syncthreads();
+    const int32_t w = s_item;
+    __syncthreads();
+    if (w >= nitems) break;
+    const PairItem it = items[w];
+    const int code = hshape[it.h];
+    double tot = epot32_part(code, S, sh, sred, A, it, false);
+    // a zero separation shows as a non-finite sum, as in epot32_kernel
+    if (__syncthreads_or(tid == 0 && !isfinite(tot))) tot = epot32_part(code, S, sh, sred, A, it, true);
     if (tid == 0) part[w] = tot;
   }
 }
@@ -1330,6 +1503,48 @@ static void add_halo_items(ItemList& L, int32_t h, int64_t n, int rows, int64_t 
   }
 }
 
+// A list of the FP32 form is cut into parts of 128 rows (rows_of(h) / 128 of
+// each item, epot32_part) when its longest item is longer than a resident
+// block's share of the pairs, for then that item runs on alone at the end, and
+// is long in itself.  A row per thread reads the tile for one row, so a list
+// that fills the device anyway is slower in parts.  epot32c of one call, whole ->
+// in parts, by longest item L and share S (pairs): 1,000 structures of 20 to
+// 200,000 members, L 16.8e6, S 3.9e6: 4.17 -> 2.04 ms; 1,500 of 20 to 2,000,000,
+// L 16.8e6, S 17.5e6: 4.48 -> 4.55; 2,000 of these, S 31e6: 6.57 -> 7.55; and
+// with shares of 0.02e6: L 6.1e6: 0.319 -> 0.284 ms, L 4.1e6: 0.235 -> 0.309.
+// A snapshot's 1,224 structures (3.7e9 pairs): 4.2 -> 2.1 ms.
+constexpr int64_t kPartMin = 5 << 20;
+
+template <class N, class F>
+static bool split_items(ItemList& L, int64_t nhalo, int blocks, N n_of, F rows_of) {
+  int64_t total = 0, longest = 0;
+  for (int64_t c : L.cost) {
+    total += c;
+    longest = std::max(longest, c);
+  }
+  if (longest < kPartMin || longest * blocks <= total) return false;
+  std::vector<PairItem> items;
+  std::vector<int64_t> cost;
+  size_t k = 0;
+  for (int64_t h = 0; h < nhalo; ++h) {
+    const int64_t end = L.hoff[h + 1];
+    const int parts = rows_of(h) / kB32;
+    L.hoff[h] = (int64_t)items.size();
+    for (; k < (size_t)end; ++k)
+      for (int p = 0; p < parts; ++p) {
+        PairItem it = L.items[k];
+        it.i0 += kB32 * p;
+        if (it.i0 >= n_of(h)) break;
+        items.push_back(it);
+        cost.push_back(L.cost[k] / parts);
+      }
+  }
+  L.hoff[nhalo] = (int64_t)items.size();
+  L.items.swap(items);
+  L.cost.swap(cost);
+  return true;
+}
+
 static void schedule(ItemList& L) {
   const int32_t ni = (int32_t)L.items.size();
   std::vector<int32_t> idx(ni);
@@ -1355,7 +1570,7 @@ struct GraphSig {
   size_t scub_bytes;
   int32_t sort_end_bit, pad2;
   int64_t nhalo;
-  int32_t n64, n32, grid64, grid32, epot, pad;
+  int32_t n64, n32, grid64, grid32, epot, parts32;
 };
 
 struct HaloEngine {
@@ -1533,7 +1748,7 @@ static int enqueue_sort32(HaloEngine& H, const HaloArgs& A, cudaStream_t s, int*
 
 // The device work of one call, in stream order; `capture` marks the timing
 // events as graph nodes.
-static int enqueue_props(HaloEngine& H, const HaloArgs& A, int64_t nhalo, int epot, int grid64, int grid32,
+static int enqueue_props(HaloEngine& H, const HaloArgs& A, int64_t nhalo, int epot, int grid64, int grid32, bool parts32,
                          cudaStream_t s, bool capture, int* launches) {
   const unsigned flags = capture ? cudaEventRecordExternal : 0u;
   AHOP_CUDA_TRY(cudaMemsetAsync(H.d_counter.p, 0, 8, s));
@@ -1582,8 +1797,12 @@ static int enqueue_props(HaloEngine& H, const HaloArgs& A, int64_t nhalo, int ep
     // the sort belongs to the FP32-compensated form and is timed with it
     int rc;
     if ((rc = enqueue_sort32(H, A, s, launches))) return rc;
-    epot32_kernel<<<grid32, kB32, 0, s>>>(A, H.l32.items.as<PairItem>(), H.d_hshape.as<int8_t>(), kDefaultShape,
-                                          H.l32.n, H.d_counter.as<int32_t>() + 1, H.l32.part.as<double>());
+    if (parts32)
+      epot32_part_kernel<<<grid32, kB32, 0, s>>>(A, H.l32.items.as<PairItem>(), H.d_hshape.as<int8_t>(), H.l32.n,
+                                                 H.d_counter.as<int32_t>() + 1, H.l32.part.as<double>());
+    else
+      epot32_kernel<<<grid32, kB32, 0, s>>>(A, H.l32.items.as<PairItem>(), H.d_hshape.as<int8_t>(), kDefaultShape,
+                                            H.l32.n, H.d_counter.as<int32_t>() + 1, H.l32.part.as<double>());
     ++*launches;
     AHOP_CUDA_TRY(cudaGetLastError());
   }
@@ -1690,6 +1909,13 @@ static int halo_run(HaloEngine& H, const AhopHaloParams* p, const int64_t* d_off
   }
   H.L64.hoff[nhalo] = (int64_t)H.L64.items.size();
   H.L32.hoff[nhalo] = (int64_t)H.L32.items.size();
+  const int grid64 = grid_for((const void*)epot64_kernel, kB64);
+  int grid32 = grid_for((const void*)epot32_kernel, kB32);
+  bool parts32 = false;
+  if (epot & 2)
+    parts32 = split_items(H.L32, nhalo, grid32, [&](int64_t h) { return h_off[h + 1] - h_off[h]; },
+                          [&](int64_t h) { return rows32_of(hshape[h]); });
+  if (parts32) grid32 = grid_for((const void*)epot32_part_kernel, kB32);
   schedule(H.L64);
   schedule(H.L32);
   AHOP_CUDA_TRY(H.d_mp1.ensure(std::max<size_t>(mch.size() * sizeof(MomP1), 16)));
@@ -1699,8 +1925,6 @@ static int halo_run(HaloEngine& H, const AhopHaloParams* p, const int64_t* d_off
   if ((rc = upload_list(H.l64, H.L64, st))) return rc;
   if ((rc = upload_list(H.l32, H.L32, st))) return rc;
   if ((rc = upload(H.d_hshape, hshape, st))) return rc;
-  const int grid64 = grid_for((const void*)epot64_kernel, kB64);
-  const int grid32 = grid_for((const void*)epot32_kernel, kB32);
   // the launches run on the engine's stream after everything queued on st
   AHOP_CUDA_TRY(cudaEventRecord(H.ev_in, st));
   AHOP_CUDA_TRY(cudaStreamWaitEvent(H.gs, H.ev_in, 0));
@@ -1721,6 +1945,7 @@ static int halo_run(HaloEngine& H, const AhopHaloParams* p, const int64_t* d_off
     sig.sort_end_bit = H.sort_end_bit;
     sig.nhalo = nhalo; sig.n64 = H.l64.n; sig.n32 = H.l32.n; sig.grid64 = grid64; sig.grid32 = grid32;
     sig.epot = epot;
+    sig.parts32 = parts32;
     if (H.gexec && memcmp(&sig, &H.gsig, sizeof sig) == 0) {
       ++H.graph_replays;
       launches = H.t.kernel_launches;
@@ -1729,14 +1954,14 @@ static int halo_run(HaloEngine& H, const AhopHaloParams* p, const int64_t* d_off
       // first call with these arguments: a capture and an instantiation cost
       // more than the ten launches they save (props of 200 halos on new arrays:
       // 0.65 -> 0.45 ms); the next call with the same ones captures
-      if ((rc = enqueue_props(H, A, nhalo, epot, grid64, grid32, H.gs, false, &launches))) return rc;
+      if ((rc = enqueue_props(H, A, nhalo, epot, grid64, grid32, parts32, H.gs, false, &launches))) return rc;
       H.last_sig = sig;
       H.graph_replays = 0;
     } else {
       if (H.gexec) { cudaGraphExecDestroy(H.gexec); H.gexec = nullptr; }
       cudaGraph_t g = nullptr;
       AHOP_CUDA_TRY(cudaStreamBeginCapture(H.gs, cudaStreamCaptureModeThreadLocal));
-      rc = enqueue_props(H, A, nhalo, epot, grid64, grid32, H.gs, true, &launches);
+      rc = enqueue_props(H, A, nhalo, epot, grid64, grid32, parts32, H.gs, true, &launches);
       const cudaError_t ec = cudaStreamEndCapture(H.gs, &g);
       if (rc) { if (g) cudaGraphDestroy(g); return rc; }
       AHOP_CUDA_TRY(ec);
@@ -1748,7 +1973,7 @@ static int halo_run(HaloEngine& H, const AhopHaloParams* p, const int64_t* d_off
       AHOP_CUDA_TRY(cudaGraphLaunch(H.gexec, H.gs));
     }
   } else {
-    if ((rc = enqueue_props(H, A, nhalo, epot, grid64, grid32, H.gs, false, &launches))) return rc;
+    if ((rc = enqueue_props(H, A, nhalo, epot, grid64, grid32, parts32, H.gs, false, &launches))) return rc;
   }
   int herr = 0;
   AHOP_CUDA_TRY(cudaMemcpyAsync(&herr, H.d_err.p, 4, cudaMemcpyDeviceToHost, H.gs));

@@ -15,8 +15,7 @@
 // their previous relative order inside.  Components are found over the saddle
 // edges > rhot (listed once per task) with labels or a union-find that link to
 // the smaller position, then reordered by a chunked stable radix sort on the
-// root.  The
-// structure can only change when rhot crosses a saddle value or a group peak
+// root.  The structure can only change when rhot crosses a saddle value or a group peak
 // density of the task, so this pass is skipped at levels below the next such
 // value.
 //
