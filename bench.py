@@ -44,12 +44,12 @@ PARAMS = dict(nvoisins=32, nhop=16, rho_threshold=80.0, fudge=4.0, fudgepsilon=1
 WORKLOAD = dict(name="c2_256cubed", npart=16_777_216, nhalo=19_200, seed=2, nmin=20, nmax=2_000_000)
 WARM_SAMPLE = dict(name="64cubed_same_generator", npart=262_144, nhalo=300, seed=2, nmax=31_250)
 
-# ncu counters of knn_leaf_kernel (DRAM read + write bytes and warp
+# ncu counters of the kNN kernels of one call (DRAM read + write bytes and warp
 # instructions, per particle) from the capture summarised in
-# profiles/knn_leaf_kernel_8m.md; the bench line scales them to the workload.
+# profiles/knn_kernels_8m.md; the bench line scales them to the workload.
 # They are re-measured whenever the kernel changes.
 NCU_KNN = dict(profiled="knn_collect, knn_finish and knn_query kernels, 8,000,000-particle clustered box, one call",
-               dram_bytes_per_particle=518.172928, warp_instructions_per_particle=1626.264373)
+               dram_bytes_per_particle=502.951136, warp_instructions_per_particle=1636.791455)
 
 
 def _gen(spec):
