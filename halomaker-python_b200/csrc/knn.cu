@@ -280,6 +280,14 @@ __device__ __forceinline__ void leaf_insert(const KnnArgs& A, WarpList& L, int32
   }
   unsigned mask = __ballot_sync(0xffffffffu, v && d <= L.r2);
   if (!mask) return;
+  const double last = __shfl_sync(0xffffffffu, L.ld, nvv - 1);
+  const bool even = v && d == last && d < CUDART_INF;
+  if (__any_sync(0xffffffffu, even)) {
+    // ties with the last entry: only those before it by particle index go in
+    // (a clump of many coincident particles is all ties)
+    const int32_t lo = A.orig[__shfl_sync(0xffffffffu, L.ls, nvv - 1)];
+    mask &= ~__ballot_sync(0xffffffffu, even && A.orig[p] > lo);
+  }
   while (mask) {
     const int src = __ffs(mask) - 1;
     const double cd = __shfl_sync(0xffffffffu, d, src);
@@ -305,7 +313,9 @@ __device__ __forceinline__ void leaf_insert(const KnnArgs& A, WarpList& L, int32
 }
 
 // Per-query depth-first traversal from the root, nearest child first (queries
-// that the lane-per-query path hands over).
+// that the lane-per-query path hands over).  A box at exactly the bound is
+// entered: the boxes are padded, so that happens only at distance 0, where
+// coincident particles beyond the nv-th are settled by particle index.
 template <int C>
 __device__ void query_dfs(const KnnArgs& A, WarpList& L, int64_t s, double qx, double qy, double qz, int lane,
                           int32_t* s_node, double* s_bd) {
@@ -319,7 +329,7 @@ __device__ void query_dfs(const KnnArgs& A, WarpList& L, int64_t s, double qx, d
     const int32_t ent = s_node[sp];
     const double bd = s_bd[sp];
     __syncwarp();
-    if (!(bd < L.r2)) continue;
+    if (!(bd <= L.r2)) continue;
     const int lvl = ent >> 27;
     const int64_t j = ent & ((1 << 27) - 1);
     if (lvl == 0) {
@@ -330,7 +340,7 @@ __device__ void query_dfs(const KnnArgs& A, WarpList& L, int64_t s, double qx, d
     const bool valid = c < A.lev_cnt[lvl - 1];
     double bdc = CUDART_INF;
     if (valid) bdc = box_dist2(A.box + 6 * (A.lev_off[lvl - 1] + c), qx, qy, qz, A.Lx, A.Ly, A.Lz);
-    const bool cand = valid && bdc < L.r2;
+    const bool cand = valid && bdc <= L.r2;
     const unsigned mask = __ballot_sync(0xffffffffu, cand);
     if (!mask) continue;
     const int cnt = __popc(mask);
@@ -347,12 +357,13 @@ __device__ void query_dfs(const KnnArgs& A, WarpList& L, int64_t s, double qx, d
       if (ob < best || (ob == best && ol < bl)) { best = ob; bl = ol; }
     }
     if (cand) {
+      // the nearest on top, the others below it in Morton order
       int r = __popc(mask & ((1u << lane) - 1));
       int slot;
       if (lane == bl) slot = sp + cnt - 1;
       else {
         int rb = __popc(mask & ((1u << bl) - 1));
-        slot = sp + (r < rb ? r : r - 1);
+        slot = sp + cnt - 2 - (r < rb ? r : r - 1);
       }
       s_node[slot] = ((lvl - 1) << 27) | (int32_t)c;
       s_bd[slot] = bdc;
