@@ -159,10 +159,13 @@ __global__ void __launch_bounds__(kAB, 6) density_adjoint_kernel(AdjArgs A, cons
   const int64_t i0 = blockIdx.x * (int64_t)kAB + (threadIdx.x & ~31), i = i0 + lane;
   if (i0 >= A.n) return;
   const double g = i < A.n ? gdens[i] : 0.0;
+  // a particle without an upstream gradient (and a lane past the end) adds
+  // nothing and reads none of its neighbours, whatever its position and list hold
   const bool act = g != 0.0;  // (NaN: yes)
+  if (!__any_sync(0xffffffffu, act)) return;
   const double C = A.xyzlong / (double)3.141592654f;
-  const double4 me = particle<kPacked>(A, i < A.n ? i : A.n - 1);
-  const int64_t jl = i < A.n ? A.nei[(size_t)A.nv * i + A.nv - 1] : 0;
+  const double4 me = particle<kPacked>(A, act ? i : 0);
+  const int64_t jl = act ? A.nei[(size_t)A.nv * i + A.nv - 1] : 0;
   const double4 last = particle<kPacked>(A, jl);
   const double lx = pdelta(me.x, last.x, A.Lx), ly = pdelta(me.y, last.y, A.Ly), lz = pdelta(me.z, last.z, A.Lz);
   const double dlast = sqrt(lx * lx + ly * ly + lz * lz);
@@ -175,7 +178,7 @@ __global__ void __launch_bounds__(kAB, 6) density_adjoint_kernel(AdjArgs A, cons
     const int m = min(32, A.nv - 1 - k0);
 #pragma unroll 4
     for (int k = 0; k < m; ++k) {
-      const int64_t j = tile[lane][k];
+      const int64_t j = act ? tile[lane][k] : 0;
       const double4 q = particle<kPacked>(A, j);
       const double dx = pdelta(me.x, q.x, A.Lx), dy = pdelta(me.y, q.y, A.Ly), dz = pdelta(me.z, q.z, A.Lz);
       const double d2 = dx * dx + dy * dy + dz * dz;
@@ -185,16 +188,18 @@ __global__ void __launch_bounds__(kAB, 6) density_adjoint_kernel(AdjArgs A, cons
       S += q.w * spline(u);
       const double wm = q.w * spline_deriv(u);
       T += wm * d;
-      const double a = act && d2 > 0.0 ? w4 * wm * id : 0.0;  // times the separation vector = times e_k
-      const double vx = a * dx, vy = a * dy, vz = a * dz;
+      const bool use = act && d2 > 0.0;  // selects the products: 0 times an infinite separation is no zero
+      const double a = w4 * wm * id;     // times the separation vector = times e_k
+      const double vx = use ? a * dx : 0.0, vy = use ? a * dy : 0.0, vz = use ? a * dz : 0.0;
       gi0 -= vx; gi1 -= vy; gi2 -= vz;
       scatter_add(gpos, j, vx, vy, vz, lane, s_v[wib], s_j[wib]);
     }
   }
   // through r = d_last / 2
   const double drho_dr = C * (-T / (r4 * r) - 3.0 * S / r4);  // d rho / d r = C [-T/r^5 - 3 S/r^4]
-  const double a = act && dlast > 0.0 ? g * 0.5 * drho_dr / dlast : 0.0;
-  const double vx = a * lx, vy = a * ly, vz = a * lz;
+  const bool use = act && dlast > 0.0;
+  const double a = g * 0.5 * drho_dr / dlast;
+  const double vx = use ? a * lx : 0.0, vy = use ? a * ly : 0.0, vz = use ? a * lz : 0.0;
   scatter_add(gpos, jl, vx, vy, vz, lane, s_v[wib], s_j[wib]);
   scatter_add(gpos, i, gi0 - vx, gi1 - vy, gi2 - vz, lane, s_v[wib], s_j[wib]);
 }
