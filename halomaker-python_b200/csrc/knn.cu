@@ -455,6 +455,8 @@ constexpr int kCollect = 48;       // particles collected per query (beyond: per
 constexpr int kWindows = 6;        // times the bins of a query are laid lower or cut finer
 constexpr int kChunkLeaves = 1 << 18;  // query leaves per pair of launches (1.6 GB of collected slots)
 static_assert((kBatch & (kBatch - 1)) == 0, "the candidate sort pads to a power of two");
+// leaves (level 0) are listed and the root (at most level kMaxLevels - 1) is popped alone
+static_assert((kMaxLevels - 3) * (kFan - 1) + kFan <= kTravStack, "the traversal's nodes fit the stack");
 
 // Shared memory of a warp of the collect kernel, 8.5 KB:
 //   bins  [bin][lane]                        A to C
@@ -1022,7 +1024,7 @@ __global__ void __launch_bounds__(kKnnWarps * 32, kKnnBlocks) knn_collect_kernel
               }
               ncand += cnt;
             } else {
-              if (sp + cnt > kStack) { whole = true; break; }
+              if (sp + cnt > kTravStack) { whole = true; break; }
               if (mine) sstack[sp + r] = ((lvl - 1) << 27) | (int32_t)c;
               sp += cnt;
             }
