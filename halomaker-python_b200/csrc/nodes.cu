@@ -213,11 +213,11 @@ __device__ __forceinline__ int32_t count_above_at(const TreeArgs& A, int32_t g, 
   while (lo < 0) {
     double v[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = j - (1 << k) >= 0 ? r[j - (1 << k)] : DBL_MAX;
+    for (int k = 0; k < 8; ++k) v[k] = j - (1 << k) >= 0 ? r[j - (1 << k)] : nan("");
     int k = 0;
 #pragma unroll
-    for (int t = 7; t >= 0; --t) k = v[t] > rhot ? t : k;  // the nearest probe above rhot
-    if (v[7] > rhot) {
+    for (int t = 7; t >= 0; --t) k = !(v[t] <= rhot) ? t : k;  // the nearest probe above rhot
+    if (!(v[7] <= rhot)) {  // before the first member counts as above, whatever rhot: the loop ends
       lo = max(0, j - (1 << k) + 1);
       if (k > 0) j -= 1 << (k - 1);
     } else {
