@@ -150,22 +150,19 @@ int stage_sort_and_tree(Engine& E, const double* d_pos, const double* d_mass) {
   morton_kernel<<<grid, T, 0, st>>>(d_pos, n, P.xlong, P.ylong, P.zlong, E.d_key.as<unsigned long long>(),
                                     E.d_idx.as<int32_t>());
   AHOP_CUDA_TRY(cudaGetLastError());
-  // Key bits that order leaves: per axis eight levels below the mean spacing
-  // (an overdensity of 2^24); the order below that only shapes the leaves'
-  // boxes, and every eight bits left out are a pass over the keys (16.7M
-  // particles: 6 passes instead of 8, sort and boxes 3.37 -> 2.95 ms).
-  int levels = 8;
-  while ((int64_t)1 << (3 * (levels - 8)) < n) ++levels;
-  const int begin_bit = std::max(0, 63 - 3 * levels);
+  // All 63 key bits: the low ones order the leaves of clumps far smaller than
+  // the mean spacing (a clump 1e-5 of the box across, 200,000 particles: kNN
+  // 144.8 ms with the bits below 2^-8 of the mean spacing left out, 1.2 with
+  // all of them, for two radix passes of eight)
   size_t tmp = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, tmp, E.d_key.as<unsigned long long>(),
                                   E.d_key2.as<unsigned long long>(), E.d_idx.as<int32_t>(),
-                                  E.d_idx2.as<int32_t>(), (int)n, begin_bit, 63, st);
+                                  E.d_idx2.as<int32_t>(), (int)n, 0, 63, st);
   AHOP_CUDA_TRY(E.d_cub.ensure(tmp));
   E.cub_calls++;
   AHOP_CUDA_TRY(cub::DeviceRadixSort::SortPairs(E.d_cub.p, tmp, E.d_key.as<unsigned long long>(),
                                                 E.d_key2.as<unsigned long long>(), E.d_idx.as<int32_t>(),
-                                                E.d_idx2.as<int32_t>(), (int)n, begin_bit, 63, st));
+                                                E.d_idx2.as<int32_t>(), (int)n, 0, 63, st));
   E.launches++;
   if (E.mass_pending) {  // host path: the masses were uploaded on the copy stream
     AHOP_CUDA_TRY(cudaStreamWaitEvent(st, E.ev_mass, 0));
