@@ -809,7 +809,8 @@ __global__ void __launch_bounds__(kKnnWarps * 32, kKnnBlocks) knn_collect_kernel
     for (int b = 0; b < kBins; ++b) col[b * 32] = 0u;
     __syncwarp();
     // whole octaves, the 31 up to 4 L^2 and one for "farther" (no particle
-    // there); a lane with nv + 1 in the lowest looks 31 octaves lower
+    // there); a lane with nv + 1 in the lowest looks 30 octaves lower, where
+    // that one is the highest
     int oct = 0, obase = A.obase;
     for (bool lower = true; lower;) {
       tile_dist(A, q, seed, seed + 96, seed + 192, nt, false,
@@ -828,7 +829,7 @@ __global__ void __launch_bounds__(kKnnWarps * 32, kKnnBlocks) knn_collect_kernel
         if (cum < need) oct = b + 1;
       }
       const bool low = oct == 0 && obase > 0;
-      if (low) obase -= kBins - 1;
+      if (low) obase -= kBins - 2;
       lower = __any_sync(0xffffffffu, low);
     }
     bool whole = !inbox || __any_sync(0xffffffffu, oct >= kBins - 1);  // the per-query search for the whole leaf
