@@ -896,6 +896,7 @@ __global__ void __launch_bounds__(kKnnWarps * 32, kKnnBlocks) knn_collect_kernel
     long long t_b = t_a, t_c = t_a, c_cand = 0;
     int cnt = 0;  // collected particles
     int nvis = 0, ncand_all = 0, npop = 0;
+    int window = 0;  // 0: counting candidates, then the number of times bins were laid lower or finer
     unsigned ntest = 0, nread = 0;
     if (!whole) {
       // Walks a list of leaves in chunks of 32: tests each leaf's box against
@@ -982,7 +983,6 @@ __global__ void __launch_bounds__(kKnnWarps * 32, kKnnBlocks) knn_collect_kernel
       __syncwarp();
       unsigned lim_kept = 0u;
       float bnd_kept = 0.f;
-      int window = 0;       // 0: counting candidates, then the number of times bins were laid lower
       bool again = false;   // this lane counts in the current lower window
       for (;;) {
         const int32_t* list = svis;
@@ -1145,6 +1145,7 @@ __global__ void __launch_bounds__(kKnnWarps * 32, kKnnBlocks) knn_collect_kernel
       atomicAdd(&A.kstats[2], (unsigned long long)nvis);
       atomicAdd(&A.kstats[8], (unsigned long long)ntest);
       atomicAdd(&A.kstats[9], (unsigned long long)nread);
+      atomicAdd(&A.kstats[10], (unsigned long long)window);
       if (whole) atomicAdd(&A.kstats[4], 1ULL);
       atomicAdd(&A.kstats[whole ? 6 : 7], (unsigned long long)(t_e - t_0));
       if (!whole) {
