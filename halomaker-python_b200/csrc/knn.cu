@@ -228,7 +228,6 @@ struct KnnArgs {
   float gpad;   // padding of a box of queries rounded to float
   float near;   // 0.49 of the smallest box length
   int obase;    // float exponent of the lowest octave bin: the 31 octaves up to 4 (largest box length)^2
-  int inbox;    // 0: box lengths whose squares leave the range of floats (per-query search only)
   int* err;     // error flag (stack overflow)
   int* next;    // next query leaf of the chunk to take
   int leaf0, nchunk;  // query leaves [leaf0, leaf0 + nchunk) of this pair of launches
@@ -399,19 +398,32 @@ __device__ __forceinline__ void finish_query(const KnnArgs& A, const WarpList& L
 // float, half width widened to cover that rounding plus every rounding of the
 // FP32 test below (2^-21 L), so the FP32 distance is never above the exact
 // point-to-box distance: a pruning bound, looser by a negligible margin.
-__global__ void leaf_box32_kernel(const double* __restrict__ box, int64_t nleaf, double Lmax,
-                                  float4* __restrict__ out) {
+// The centre's w: twice what the node's pairs can be apart beyond a box length
+// on some axis (the boxes' padding, for one); the reference's distance is 0
+// there, which only the per-query search takes, so beyond 1e-9 of the box it
+// is +inf (a particle outside the box, and the leaves across the box from it),
+// as where FP32 coordinates or distances would be too coarse (inbox = 0, or
+// particles outside [-L, L]).
+__global__ void leaf_box32_kernel(const double* __restrict__ box, int64_t nbox, double Lx, double Ly, double Lz,
+                                  int inbox, float4* __restrict__ out) {
   const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (j >= nleaf) return;
+  if (j >= nbox) return;
   const double* b = box + 6 * j;
-  const double pad = Lmax * 0x1p-21;
+  const double* root = box + 6 * (nbox - 1);
+  const double L[3] = {Lx, Ly, Lz};
+  const double pad = fmax(Lx, fmax(Ly, Lz)) * 0x1p-21;
   float c[3], w[3];
+  double over = 0.0;
+  bool in = inbox;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     c[k] = (float)b[k];
     w[k] = __double2float_ru(b[3 + k] + fabs(b[k] - (double)c[k]) + pad);
+    in = in && fabs(root[k]) + root[3 + k] <= 1.001 * L[k];  // (the pad aside)
+    over = fmax(over, fabs(b[k] - root[k]) + b[3 + k] + root[3 + k] - L[k]);
   }
-  out[2 * j] = make_float4(c[0], c[1], c[2], 0.f);
+  in = in && over <= 1e-9 * fmin(Lx, fmin(Ly, Lz));
+  out[2 * j] = make_float4(c[0], c[1], c[2], in ? __double2float_ru(2.0 * over) : CUDART_INF_F);
   out[2 * j + 1] = make_float4(w[0], w[1], w[2], 0.f);
 }
 
@@ -430,6 +442,7 @@ constexpr int kKnnWarps = 4;       // warps per block
 constexpr int kKnnBlocks = 6;      // collect: blocks per SM (80 registers, 8.5 KB of shared memory per warp)
 constexpr int kFinWarps = 4;       // finish: warps per block
 constexpr int kFinBlocks = 5;      // finish: blocks per SM
+constexpr int kLostBlocks = 16;    // blocks per SM for the queries left over: usually few, at times whole chunks
 constexpr int kBatch = 256;        // candidate leaves sorted and counted at a time
 constexpr int kVisMax = 160;       // counted leaves per query leaf, three times the mean; beyond, a warp for each
                                    // of the 32 queries is as cheap and ends sooner (262,144 particles: 1.15-1.29
@@ -752,12 +765,6 @@ __global__ void __launch_bounds__(kKnnWarps * 32, kKnnBlocks) knn_collect_kernel
   float4* const sbox = reinterpret_cast<float4*>(W + kOffBox);
   Group* const sgroup = reinterpret_cast<Group*>(W + kOffGroup);
   int32_t* const svis = reinterpret_cast<int32_t*>(W + kOffVis);
-  // positions outside the box: only the per-query search has the reference's
-  // distances there
-  const double* rb = A.box + 6 * A.lev_off[top];
-  const bool inbox = A.inbox && fabs(rb[0]) + rb[3] <= 0.5 * A.Lx * (1.0 + 1e-9) &&
-                     fabs(rb[1]) + rb[4] <= 0.5 * A.Ly * (1.0 + 1e-9) &&
-                     fabs(rb[2]) + rb[5] <= 0.5 * A.Lz * (1.0 + 1e-9);
   for (;;) {
     int jl = 0;
     if (lane == 0) jl = atomicAdd(A.next, 1);
@@ -784,7 +791,9 @@ __global__ void __launch_bounds__(kKnnWarps * 32, kKnnBlocks) knn_collect_kernel
     // margins of widen()
     const float amax = __uint_as_float(__reduce_max_sync(
         0xffffffffu, __float_as_uint(fmaxf(fabsf(lx), fmaxf(fabsf(ly), fabsf(lz))))));
-    const float eabs2 = 0x1p-19f * amax + A.eabs2;
+    const float beyond = A.box32[2 * (int64_t)jl].w;  // pairs more than a box length apart (leaf_box32_kernel)
+    const float eabs2 = 0x1p-19f * amax + A.eabs2 + beyond;
+    bool whole = !(beyond < CUDART_INF_F);  // the per-query search for the whole leaf
     // a bound on FP32 distances -> a bound on exact ones, and back: (sqrt(e)
     // (1 + 2^-19) + 2 eabs)^2 covers both steps
     auto widen = [&](float e2) {
@@ -812,7 +821,7 @@ __global__ void __launch_bounds__(kKnnWarps * 32, kKnnBlocks) knn_collect_kernel
     // there); a lane with nv + 1 in the lowest looks 30 octaves lower, where
     // that one is the highest
     int oct = 0, obase = A.obase;
-    for (bool lower = true; lower;) {
+    for (bool lower = !whole; lower;) {
       tile_dist(A, q, seed, seed + 96, seed + 192, nt, false,
                 [&](int, unsigned k0, unsigned k1, unsigned k2, unsigned k3) {
                   atomicAdd(&col[min(max((int)(k0 >> 23) - obase, 0), kBins - 1) * 32], 1u);
@@ -832,7 +841,7 @@ __global__ void __launch_bounds__(kKnnWarps * 32, kKnnBlocks) knn_collect_kernel
       if (low) obase -= kBins - 2;
       lower = __any_sync(0xffffffffu, low);
     }
-    bool whole = !inbox || __any_sync(0xffffffffu, oct >= kBins - 1);  // the per-query search for the whole leaf
+    whole |= __any_sync(0xffffffffu, oct >= kBins - 1);
     unsigned lim = (unsigned)(obase + oct + 1) << 23;  // float bits: upper edge, exclusive
     int shift = kBinShift;
     int wbase = (int)(lim >> shift) - kBins;      // bin b: bits [(wbase + b) << shift, (wbase + b + 1) << shift)
@@ -1201,8 +1210,8 @@ __global__ void __launch_bounds__(kFinWarps * 32, kFinBlocks) knn_finish_kernel(
 
 // One warp per query: the queries of a chunk that the lane-per-query kernels
 // left over (kAll false), below the bound they have, or every query of a small
-// set (kAll), below the (nv+1)-th distance (to 8 bits) among the particles of
-// its own and the two adjacent leaves.
+// set (kAll) and those left without a bound, below the (nv+1)-th distance (to 8
+// bits) among the particles of its own and the two adjacent leaves.
 template <int C, bool kAll>
 __global__ void __launch_bounds__(kFinWarps * 32) knn_query_kernel(KnnArgs A) {
   __shared__ double s_bd[kFinWarps][kStack];
@@ -1212,14 +1221,14 @@ __global__ void __launch_bounds__(kFinWarps * 32) knn_query_kernel(KnnArgs A) {
   const int nvv = C ? C : A.nv;
   for (int i = blockIdx.x * kFinWarps + wib; i < nq; i += gridDim.x * kFinWarps) {
     int32_t s = i;
-    double cap;
+    double cap = CUDART_INF;
     if (!kAll) {
       const int at = A.lost[i];
       s = A.leaf0 * kLeaf + at;
       cap = (double)__uint_as_float((unsigned)A.coll[(size_t)(at >> 5) * (kCollect * 32) + (at & 31)]);
     }
     const double4 p = A.p4[s];
-    if (kAll) {
+    if (kAll || !(cap < CUDART_INF)) {
       unsigned k[3];
 #pragma unroll
       for (int t = 0; t < 3; ++t) {
@@ -1264,20 +1273,19 @@ int stage_knn_density(Engine& E) {
   const int64_t nbox = E.lev_off[E.nlev];  // boxes of every level
   AHOP_CUDA_TRY(E.d_box32.ensure((size_t)nbox * 32 + 32));
   A.box32 = E.d_box32.as<float4>();
+  const double Lmin = std::min(P.xlong, std::min(P.ylong, P.zlong)), Lmax = std::max(P.xlong, std::max(P.ylong, P.zlong));
   E.launches++;
   leaf_box32_kernel<<<(unsigned)((nbox + 255) / 256), 256, 0, E.stream>>>(
-      A.box, nbox, std::max(P.xlong, std::max(P.ylong, P.zlong)), E.d_box32.as<float4>());
+      A.box, nbox, P.xlong, P.ylong, P.zlong, Lmax < 1e15 && Lmin > 1e-15, E.d_box32.as<float4>());
   AHOP_CUDA_TRY(cudaGetLastError());
   for (int l = 0; l < kMaxLevels; ++l) { A.lev_off[l] = E.lev_off[l]; A.lev_cnt[l] = E.lev_cnt[l]; }
   A.nlev = E.nlev;
   A.n = n;
   A.n32 = (int32_t)n;
   A.Lx = P.xlong; A.Ly = P.ylong; A.Lz = P.zlong; A.xyzlong = P.xyzlong;
-  const double Lmin = std::min(P.xlong, std::min(P.ylong, P.zlong)), Lmax = std::max(P.xlong, std::max(P.ylong, P.zlong));
   A.eabs2 = (float)(0x1p-45 * Lmax);
   A.gpad = (float)(0x1p-22 * Lmax);
   A.near = (float)(0.49 * Lmin);
-  A.inbox = Lmax < 1e15 && Lmin > 1e-15;
   {
     const float l2 = (float)(4.0 * Lmax * Lmax);
     uint32_t bits;
@@ -1331,7 +1339,7 @@ int stage_knn_density(Engine& E) {
     const int64_t want = (A.nchunk + kKnnWarps - 1) / kKnnWarps;
     kcol<<<(unsigned)std::min((int64_t)nsm * per_sm, want), kKnnWarps * 32, smem, E.stream>>>(A);
     kfin<<<(unsigned)((A.nchunk + kFinWarps - 1) / kFinWarps), kFinWarps * 32, 0, E.stream>>>(A);
-    const unsigned lgrid = (unsigned)std::min<int64_t>(nsm * 4, (A.nchunk * 32 + kFinWarps - 1) / kFinWarps);
+    const unsigned lgrid = (unsigned)std::min<int64_t>(nsm * kLostBlocks, (A.nchunk * 32 + kFinWarps - 1) / kFinWarps);
     if (nv32) knn_query_kernel<32, false><<<lgrid, kFinWarps * 32, 0, E.stream>>>(A);
     else knn_query_kernel<0, false><<<lgrid, kFinWarps * 32, 0, E.stream>>>(A);
     AHOP_CUDA_TRY(cudaGetLastError());
