@@ -30,6 +30,7 @@
 #include <cmath>
 #include <cstdint>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -417,20 +418,64 @@ struct Packed {
   ~Packed() { if (p) cudaFreeAsync(p, st); }
 };
 
-// Items, tiles and partial sums of ahop_epot_grad, kept between calls; one call
-// at a time uses them (the call waits for its kernels).  Buffers beyond
-// kGradKeep go back at the end of the call.
+// Items, tiles and partial sums of ahop_epot_grad, kept between calls.  A call
+// takes an idle set of its device, or a new one while others are in use on
+// other threads or streams, and gives it back when its kernels are done; up to
+// kGradKeep bytes of idle sets stay.
 constexpr size_t kGradKeep = (size_t)256 << 20;
 struct GradWork {
-  std::mutex m;
   int device = -1;
   DevBuf items, tiles, part;
+  GradWork* next = nullptr;
+  size_t bytes() const { return items.bytes + tiles.bytes + part.bytes; }
   void release() { items.release(); tiles.release(); part.release(); }
 };
-static GradWork& grad_work() {
-  static GradWork* w = new GradWork();
-  return *w;
+struct GradPool {
+  std::mutex m;
+  GradWork* idle = nullptr;
+  size_t bytes = 0;  // of the idle sets
+};
+static GradPool& grad_pool() {
+  static GradPool* p = new GradPool();
+  return *p;
 }
+
+struct GradLease {
+  GradWork* w = nullptr;
+  cudaStream_t st = nullptr;
+  bool done = false;  // the kernels that use the set have ended
+  bool take(int device, cudaStream_t s) {
+    st = s;
+    GradPool& P = grad_pool();
+    std::lock_guard<std::mutex> g(P.m);
+    for (GradWork** at = &P.idle; *at; at = &(*at)->next)
+      if ((*at)->device == device) {
+        w = *at;
+        *at = w->next;
+        P.bytes -= w->bytes();
+        return true;
+      }
+    w = new (std::nothrow) GradWork();
+    if (w) w->device = device;
+    return w != nullptr;
+  }
+  ~GradLease() {
+    if (!w) return;
+    if (!done) cudaStreamSynchronize(st);
+    GradPool& P = grad_pool();
+    {
+      std::lock_guard<std::mutex> g(P.m);
+      if (P.bytes + w->bytes() <= kGradKeep) {
+        P.bytes += w->bytes();
+        w->next = P.idle;
+        P.idle = w;
+        return;
+      }
+    }
+    w->release();
+    delete w;
+  }
+};
 
 void release_adjoint_memory() {
   {
@@ -439,13 +484,17 @@ void release_adjoint_memory() {
     for (cudaMemPool_t p : R.pool)
       if (p) cudaMemPoolTrimTo(p, 0);
   }
-  GradWork& w = grad_work();
-  std::lock_guard<std::mutex> g(w.m);
-  if (w.device < 0) return;
+  GradPool& P = grad_pool();
+  std::lock_guard<std::mutex> g(P.m);
   int now = 0;
   cudaGetDevice(&now);
-  cudaSetDevice(w.device);
-  w.release();
+  while (GradWork* w = P.idle) {
+    P.idle = w->next;
+    cudaSetDevice(w->device);
+    w->release();
+    delete w;
+  }
+  P.bytes = 0;
   cudaSetDevice(now);
 }
 
@@ -511,16 +560,11 @@ int ahop_epot_grad(const AhopHaloParams* p, const int64_t* d_off, const int64_t*
   }
   if (items.empty()) return AHOP_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  GradWork& W = grad_work();
-  std::lock_guard<std::mutex> guard(W.m);
   int dev = 0;
   AHOP_CUDA_TRY(cudaGetDevice(&dev));
-  if (W.device >= 0 && W.device != dev) {
-    AHOP_CUDA_TRY(cudaSetDevice(W.device));
-    W.release();
-    AHOP_CUDA_TRY(cudaSetDevice(dev));
-  }
-  W.device = dev;
+  GradLease lease;
+  if (!lease.take(dev, st)) { set_error("out of memory"); return AHOP_ENOMEM; }
+  GradWork& W = *lease.w;
   AHOP_CUDA_TRY(W.items.ensure(items.size() * sizeof(GradItem)));
   AHOP_CUDA_TRY(W.tiles.ensure(tiles.size() * sizeof(GradTile)));
   AHOP_CUDA_TRY(W.part.ensure((size_t)parts * (3 * kGT) * 8));
@@ -537,7 +581,7 @@ int ahop_epot_grad(const AhopHaloParams* p, const int64_t* d_off, const int64_t*
     AHOP_CUDA_TRY(cudaGetLastError());
   }
   AHOP_CUDA_TRY(cudaStreamSynchronize(st));
-  if (W.items.bytes + W.tiles.bytes + W.part.bytes > kGradKeep) W.release();
+  lease.done = true;
   return AHOP_OK;
 }
 
