@@ -367,6 +367,14 @@ static RowPools& row_pools() {
   return *p;
 }
 
+// The pool's calls wait for no stream, but count as unsafe beside a capture on
+// another thread, and would end it: they are made in the relaxed mode.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 struct Packed {
   void* p = nullptr;
   cudaStream_t st = nullptr;
@@ -374,6 +382,7 @@ struct Packed {
   // own the memory)
   int make(AdjArgs& A, cudaStream_t s) {
     if (A.n < kPackMin) return AHOP_OK;
+    RelaxedCapture relaxed;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     AHOP_CUDA_TRY(cudaStreamIsCapturing(s, &cs));
     if (cs != cudaStreamCaptureStatusNone) return AHOP_OK;
@@ -410,12 +419,13 @@ struct Packed {
   }
   int done() {
     if (!p) return AHOP_OK;
+    RelaxedCapture relaxed;
     void* q = p;
     p = nullptr;
     AHOP_CUDA_TRY(cudaFreeAsync(q, st));
     return AHOP_OK;
   }
-  ~Packed() { if (p) cudaFreeAsync(p, st); }
+  ~Packed() { done(); }
 };
 
 // Items, tiles and partial sums of ahop_epot_grad, kept between calls.  A call
