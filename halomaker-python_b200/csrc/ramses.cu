@@ -329,13 +329,12 @@ extern "C" int ahop_ramses_open(const char* const* paths, int32_t nfiles, const 
   S.files.assign(nfiles, PartFile());
   S.paths.assign(paths, paths + nfiles);
   int rc;
-  int64_t total = 0, dev_bytes = 0, max_file = 0;
+  int64_t total = 0, dev_bytes = 0;
   for (int f = 0; f < nfiles; ++f) {
     if ((rc = walk_file(S.paths[f], p->version, S.files[f]))) return rc;
     PartFile& P = S.files[f];
     P.first = total;
     total += P.npart;
-    max_file = std::max(max_file, P.bytes);
     for (int r = 0; r < R_N; ++r) {
       P.dev[r] = -1;
       if (P.file_off[r] < 0) continue;
@@ -473,12 +472,13 @@ extern "C" int ahop_ramses_close(void) {
 namespace ahop {
 void release_reader_memory() {
   RamsesState& S = rstate();
+  S.h_stage.release();  // the uploads were waited for by ahop_ramses_open
+  if (S.open) return;   // files are open: their payloads stay until decoded and closed
   ahop_ramses_close();
   S.d_raw.release();
   S.d_files.release();
   S.d_cnt.release();
   S.d_owner.release();
   S.d_flag.release();
-  S.h_stage.release();
 }
 }  // namespace ahop

@@ -109,8 +109,10 @@ int ahop_get_timings(AhopTimings* t);
  * buffers stay cached for the next compute; ahop_release_device_memory()
  * frees them. */
 int ahop_close(void);
-/* Frees every device buffer of the finder (no reference counterpart: the
- * Fortran module has no device memory). */
+/* Frees every device buffer of the finder, and what the gradients and the
+ * part-file reader keep between calls (a reader that is open keeps its
+ * payloads until ahop_ramses_close).  No reference counterpart: the Fortran
+ * module has no device memory. */
 int ahop_release_device_memory(void);
 
 /* ---- stage views for parity tests (host copies of device intermediates) ---- */
