@@ -1614,7 +1614,8 @@ struct HaloEngine {
   cudaGraphExec_t gexec = nullptr;
   GraphSig gsig{};      // arguments of gexec
   GraphSig last_sig{};  // ... of the last call that was not a replay
-  int32_t graph_replays = 0;
+  int32_t graph_replays = 0;   // launches of gexec since its capture
+  int32_t graph_launches = 0;  // kernels in gexec
 };
 
 static HaloEngine& halo_engine() {
@@ -1940,6 +1941,7 @@ static int halo_run(HaloEngine& H, const AhopHaloParams* p, const int64_t* d_off
   AHOP_CUDA_TRY(cudaEventRecord(H.ev_in, st));
   AHOP_CUDA_TRY(cudaStreamWaitEvent(H.gs, H.ev_in, 0));
   int launches = 0;
+  int32_t replay = 0;  // which launch of the captured graph this call is (0: launched directly)
   if (H.use_graph) {
     GraphSig sig;
     memset(&sig, 0, sizeof sig);
@@ -1958,8 +1960,8 @@ static int halo_run(HaloEngine& H, const AhopHaloParams* p, const int64_t* d_off
     sig.epot = epot;
     sig.parts32 = parts32;
     if (H.gexec && memcmp(&sig, &H.gsig, sizeof sig) == 0) {
-      ++H.graph_replays;
-      launches = H.t.kernel_launches;
+      replay = ++H.graph_replays;
+      launches = H.graph_launches;
       AHOP_CUDA_TRY(cudaGraphLaunch(H.gexec, H.gs));
     } else if (memcmp(&sig, &H.last_sig, sizeof sig) != 0) {
       // first call with these arguments: a capture and an instantiation cost
@@ -1967,7 +1969,6 @@ static int halo_run(HaloEngine& H, const AhopHaloParams* p, const int64_t* d_off
       // 0.65 -> 0.45 ms); the next call with the same ones captures
       if ((rc = enqueue_props(H, A, nhalo, epot, grid64, grid32, parts32, H.gs, false, &launches))) return rc;
       H.last_sig = sig;
-      H.graph_replays = 0;
     } else {
       if (H.gexec) { cudaGraphExecDestroy(H.gexec); H.gexec = nullptr; }
       cudaGraph_t g = nullptr;
@@ -1980,7 +1981,8 @@ static int halo_run(HaloEngine& H, const AhopHaloParams* p, const int64_t* d_off
       cudaGraphDestroy(g);
       AHOP_CUDA_TRY(ei);
       H.gsig = sig;
-      H.graph_replays = 1;
+      H.graph_launches = launches;
+      replay = H.graph_replays = 1;
       AHOP_CUDA_TRY(cudaGraphLaunch(H.gexec, H.gs));
     }
   } else {
@@ -2000,7 +2002,7 @@ static int halo_run(HaloEngine& H, const AhopHaloParams* p, const int64_t* d_off
   H.t.items = H.l64.n + H.l32.n;
   H.t.kernel_launches = launches;
   H.t.tune_ms = tune_total;
-  H.t.graph_replays = H.use_graph ? H.graph_replays : -1;
+  H.t.graph_replays = H.use_graph ? replay : -1;
   return AHOP_OK;
 }
 
