@@ -46,6 +46,35 @@ static int ensure_device(Engine& E) {
   return AHOP_OK;
 }
 
+static void release_device(Engine& E) {
+  DevBuf* bufs[] = {&E.d_pos_in, &E.d_mass_in, &E.d_key, &E.d_key2, &E.d_idx, &E.d_idx2, &E.d_x, &E.d_y,
+                    &E.d_z, &E.d_m, &E.d_p4, &E.d_orig, &E.d_rank, &E.d_box, &E.d_box32, &E.d_cub, &E.d_nei, &E.d_coll, &E.d_dens,
+                    &E.d_hop, &E.d_root, &E.d_group, &E.d_peakflag, &E.d_densg, &E.d_gpeak, &E.d_goff,
+                    &E.d_gmem, &E.d_gmem_rho, &E.d_gmem_rho_pref, &E.d_sad_key, &E.d_sad_key2, &E.d_sad_val,
+                    &E.d_sad_val2, &E.d_sad_cnt, &E.d_sad_keep, &E.d_sad_kpos, &E.d_flags, &E.d_soff,
+                    &E.d_sisad, &E.d_srho, &E.d_nodes, &E.d_tree_scratch, &E.d_liste, &E.d_dens_orig,
+                    &E.d_rtab, &E.d_itab, &E.d_tprof, &E.d_pairs, &E.d_pair_sums, &E.d_node_aux,
+                    &E.d_forest, &E.d_moff, &E.d_misad, &E.d_mrho, &E.d_task_sort};
+  if (E.device >= 0) cudaSetDevice(E.device);
+  for (DevBuf* b : bufs) b->release();
+  E.h_liste.release(); E.h_dens.release(); E.h_rtab.release(); E.h_itab.release();
+}
+
+// Runs a compute; when it runs out of device memory, once more on buffers that
+// are just as large as it needs.
+template <class F>
+static int with_room(Engine& E, F&& compute) {
+  int rc = compute();
+  if (rc != AHOP_ENOMEM) return rc;
+  cudaGetLastError();
+  for (cudaStream_t s : {E.stream, E.stream2, E.stream_copy}) AHOP_CUDA_TRY(cudaStreamSynchronize(s));
+  release_device(E);
+  exact_buffers = true;
+  rc = compute();
+  exact_buffers = false;
+  return rc;
+}
+
 static int validate(const Engine& E, int64_t n) {
   const Params& P = E.prm;
   if (n <= 0) { set_error("npart must be positive"); return AHOP_EINVAL; }
@@ -204,8 +233,7 @@ int ahop_sync_others(const AhopOthers* o) {
   return AHOP_OK;
 }
 
-int ahop_compute_adaptahop_device(const double* d_pos, const double* d_mass, int64_t npart, void* stream) {
-  Engine& E = engine();
+static int compute_device(Engine& E, const double* d_pos, const double* d_mass, int64_t npart, void* stream) {
   int rc;
   if ((rc = ensure_device(E))) return rc;
   if ((rc = validate(E, npart))) return rc;
@@ -222,10 +250,13 @@ int ahop_compute_adaptahop_device(const double* d_pos, const double* d_mass, int
   return AHOP_OK;
 }
 
-int ahop_compute_adaptahop(const double* pos_in, const double* mass_in, int64_t npart) {
+int ahop_compute_adaptahop_device(const double* d_pos, const double* d_mass, int64_t npart, void* stream) {
   Engine& E = engine();
+  return with_room(E, [&] { return compute_device(E, d_pos, d_mass, npart, stream); });
+}
+
+static int compute_host(Engine& E, const double* pos_in, const double* mass_in, int64_t npart) {
   int rc;
-  if (!pos_in || !mass_in) { set_error("null input"); return AHOP_EINVAL; }
   if ((rc = ensure_device(E))) return rc;
   if ((rc = validate(E, npart))) return rc;
   E.have_result = false;
@@ -277,6 +308,12 @@ int ahop_compute_adaptahop(const double* pos_in, const double* mass_in, int64_t 
   return AHOP_OK;
 }
 
+int ahop_compute_adaptahop(const double* pos_in, const double* mass_in, int64_t npart) {
+  Engine& E = engine();
+  if (!pos_in || !mass_in) { set_error("null input"); return AHOP_EINVAL; }
+  return with_room(E, [&] { return compute_host(E, pos_in, mass_in, npart); });
+}
+
 int ahop_get_outputs(AhopOutputs* out) {
   Engine& E = engine();
   if (!out) { set_error("null out"); return AHOP_EINVAL; }
@@ -314,20 +351,6 @@ int ahop_get_timings(AhopTimings* t) {
   return AHOP_OK;
 }
 
-static void release_device(Engine& E) {
-  DevBuf* bufs[] = {&E.d_pos_in, &E.d_mass_in, &E.d_key, &E.d_key2, &E.d_idx, &E.d_idx2, &E.d_x, &E.d_y,
-                    &E.d_z, &E.d_m, &E.d_p4, &E.d_orig, &E.d_rank, &E.d_box, &E.d_box32, &E.d_cub, &E.d_nei, &E.d_coll, &E.d_dens,
-                    &E.d_hop, &E.d_root, &E.d_group, &E.d_peakflag, &E.d_densg, &E.d_gpeak, &E.d_goff,
-                    &E.d_gmem, &E.d_gmem_rho, &E.d_gmem_rho_pref, &E.d_sad_key, &E.d_sad_key2, &E.d_sad_val,
-                    &E.d_sad_val2, &E.d_sad_cnt, &E.d_sad_keep, &E.d_sad_kpos, &E.d_flags, &E.d_soff,
-                    &E.d_sisad, &E.d_srho, &E.d_nodes, &E.d_tree_scratch, &E.d_liste, &E.d_dens_orig,
-                    &E.d_rtab, &E.d_itab, &E.d_tprof, &E.d_pairs, &E.d_pair_sums, &E.d_node_aux,
-                    &E.d_forest, &E.d_moff, &E.d_misad, &E.d_mrho, &E.d_task_sort};
-  if (E.device >= 0) cudaSetDevice(E.device);
-  for (DevBuf* b : bufs) b->release();
-  E.h_liste.release(); E.h_dens.release(); E.h_rtab.release(); E.h_itab.release();
-}
-
 // close (f90:3227-3264) deallocates the module's arrays.  Here the module
 // outputs are dropped; device buffers stay cached for the next compute (a
 // pool, like torch's caching allocator) -- the reference calls close() after
@@ -355,10 +378,8 @@ int ahop_release_device_memory(void) {
 }
 
 // ---------------------------------------------------------------- debug views
-int ahop_debug_compute_stages(const double* pos_in, const double* mass_in, int64_t npart, int32_t last_stage) {
-  Engine& E = engine();
+static int compute_stages(Engine& E, const double* pos_in, const double* mass_in, int64_t npart, int32_t last_stage) {
   int rc;
-  if (!pos_in || !mass_in) { set_error("null input"); return AHOP_EINVAL; }
   if ((rc = ensure_device(E))) return rc;
   if ((rc = validate(E, npart))) return rc;
   E.have_result = false;
@@ -373,6 +394,12 @@ int ahop_debug_compute_stages(const double* pos_in, const double* mass_in, int64
   if (rc) return rc;
   AHOP_CUDA_TRY(cudaStreamSynchronize(E.stream));
   return AHOP_OK;
+}
+
+int ahop_debug_compute_stages(const double* pos_in, const double* mass_in, int64_t npart, int32_t last_stage) {
+  Engine& E = engine();
+  if (!pos_in || !mass_in) { set_error("null input"); return AHOP_EINVAL; }
+  return with_room(E, [&] { return compute_stages(E, pos_in, mass_in, npart, last_stage); });
 }
 
 int ahop_debug_tree_stats(int64_t* out, int32_t n) {

@@ -11,27 +11,17 @@
 
 namespace ahop {
 
-// Growable device buffer; never shrinks until close().  A buffer that has to
-// grow takes an eighth more (when there is room): its size follows counts that
-// differ a little from one snapshot to the next, and each growth is a
-// cudaFree and a cudaMalloc (16.7M particles: up to 20 ms of a call).
+// Growable device buffer; never shrinks until close().
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
   cudaError_t ensure(size_t need) {
     if (need <= bytes) return cudaSuccess;
-    size_t want = p ? need + need / 8 : need;
     if (p) cudaFree(p);
     p = nullptr;
     bytes = 0;
-    if (!want) want = 16;
-    cudaError_t e = cudaMalloc(&p, want);
-    if (e != cudaSuccess && want > need && need) {
-      cudaGetLastError();
-      want = need;
-      e = cudaMalloc(&p, want);
-    }
-    if (e == cudaSuccess) bytes = want;
+    cudaError_t e = cudaMalloc(&p, need ? need : 16);
+    if (e == cudaSuccess) bytes = need ? need : 16;
     else p = nullptr;
     return e;
   }
@@ -41,6 +31,24 @@ struct DevBuf {
     bytes = 0;
   }
   template <class T> T* as() const { return static_cast<T*>(p); }
+};
+
+// A buffer whose size follows counts that differ a little from one snapshot to
+// the next (groups, links, nodes): when it has to grow it takes an eighth more,
+// 32 MB at most, since each growth is a cudaFree and a cudaMalloc (262,144
+// particles: a call that grows them 10.5 ms instead of 5.3).  A call that runs
+// out of memory gives everything back and runs again without (with_room in
+// capi.cu), so that slack never takes the room of a later buffer.
+inline thread_local bool exact_buffers = false;
+struct CountBuf : DevBuf {
+  cudaError_t ensure(size_t need) {
+    if (p && need > bytes && !exact_buffers) {
+      const size_t slack = need / 8 < ((size_t)32 << 20) ? need / 8 : (size_t)32 << 20;
+      if (DevBuf::ensure(need + slack) == cudaSuccess) return cudaSuccess;
+      cudaGetLastError();
+    }
+    return DevBuf::ensure(need);
+  }
 };
 
 // Growable pinned host buffer (module outputs live here; fast D2H).
@@ -137,7 +145,7 @@ struct Engine {
   int32_t nlev = 0;
   int64_t lev_off[kMaxLevels + 1] = {};
   int64_t lev_cnt[kMaxLevels] = {};
-  DevBuf d_cub;                          // CUB scratch
+  CountBuf d_cub;                          // CUB scratch
 
   // kNN / density
   DevBuf d_nei;                          // [n][nstore] sorted-slot neighbour ids
@@ -147,34 +155,34 @@ struct Engine {
   DevBuf d_hop, d_root, d_group;         // per sorted slot
   DevBuf d_peakflag;                     // per orig index
   int32_t ngroups = 0;
-  DevBuf d_densg;                        // [ngroups+1] peak density per group
-  DevBuf d_gpeak;                        // [ngroups+1] sorted slot of peak
-  DevBuf d_goff;                         // [ngroups+2] member CSR offsets (desc orig order)
+  CountBuf d_densg;                        // [ngroups+1] peak density per group
+  CountBuf d_gpeak;                        // [ngroups+1] sorted slot of peak
+  CountBuf d_goff;                         // [ngroups+2] member CSR offsets (desc orig order)
   DevBuf d_gmem;                         // [nactive] sorted slots
-  DevBuf d_gmem_rho;                     // [nactive] member density in desc-density order
-  DevBuf d_gmem_rho_pref;                // [nactive] prefix sums of density (desc density order)
+  CountBuf d_gmem_rho;                     // [nactive] member density in desc-density order
+  CountBuf d_gmem_rho_pref;                // [nactive] prefix sums of density (desc density order)
   int64_t nactive = 0;
   // saddles
-  DevBuf d_sad_key, d_sad_key2, d_sad_val, d_sad_val2, d_sad_cnt, d_sad_keep, d_sad_kpos;
+  CountBuf d_sad_key, d_sad_key2, d_sad_val, d_sad_val2, d_sad_cnt, d_sad_keep, d_sad_kpos;
   DevBuf d_flags;                        // small device error/status flags
-  DevBuf d_soff, d_sisad, d_srho;        // final CSR
+  CountBuf d_soff, d_sisad, d_srho;        // final CSR
   int32_t nconn = 0;
   // nodes
-  DevBuf d_nodes;                        // NodeRec[nnodesmax+1]
-  DevBuf d_tree_scratch;
-  DevBuf d_task_sort;                    // wave task ordering scratch
+  CountBuf d_nodes;                        // NodeRec[nnodesmax+1]
+  CountBuf d_tree_scratch;
+  CountBuf d_task_sort;                    // wave task ordering scratch
   DevBuf d_tprof;                        // per-task profile rows (debug)
-  DevBuf d_forest;                       // saddle-forest scratch
-  DevBuf d_moff, d_misad, d_mrho;        // saddle forest CSR (rows by decreasing saddle)
+  CountBuf d_forest;                       // saddle-forest scratch
+  CountBuf d_moff, d_misad, d_mrho;        // saddle forest CSR (rows by decreasing saddle)
   int32_t* m_isad = nullptr;             // sorted forest rows inside d_misad / d_mrho
   double* m_rho = nullptr;
-  DevBuf d_pairs;                        // (node, group) pair keys, sort double buffer
-  DevBuf d_pair_sums;                    // [npairs][8] per-pair sums
-  DevBuf d_node_aux;                     // per node: pair range, posref
+  CountBuf d_pairs;                        // (node, group) pair keys, sort double buffer
+  CountBuf d_pair_sums;                    // [npairs][8] per-pair sums
+  CountBuf d_node_aux;                     // per node: pair range, posref
   int32_t nnodes = 0;
   DevBuf d_liste;                        // [n] node id per ORIG particle (1-based), 0 none
   DevBuf d_dens_orig;                    // [n] density in ORIG order
-  DevBuf d_rtab, d_itab;                 // exported tables
+  CountBuf d_rtab, d_itab;                 // exported tables
 
   // host copies (module outputs), pinned
   HostBuf h_liste, h_itab, h_dens, h_rtab;
