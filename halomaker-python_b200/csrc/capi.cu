@@ -47,14 +47,13 @@ static int ensure_device(Engine& E) {
 }
 
 static void release_device(Engine& E) {
-  DevBuf* bufs[] = {&E.d_pos_in, &E.d_mass_in, &E.d_key, &E.d_key2, &E.d_idx, &E.d_idx2, &E.d_x, &E.d_y,
-                    &E.d_z, &E.d_m, &E.d_p4, &E.d_orig, &E.d_rank, &E.d_box, &E.d_box32, &E.d_cub, &E.d_nei, &E.d_coll, &E.d_dens,
-                    &E.d_hop, &E.d_root, &E.d_group, &E.d_peakflag, &E.d_densg, &E.d_gpeak, &E.d_goff,
-                    &E.d_gmem, &E.d_gmem_rho, &E.d_gmem_rho_pref, &E.d_sad_key, &E.d_sad_key2, &E.d_sad_val,
-                    &E.d_sad_val2, &E.d_sad_cnt, &E.d_sad_keep, &E.d_sad_kpos, &E.d_flags, &E.d_soff,
-                    &E.d_sisad, &E.d_srho, &E.d_nodes, &E.d_tree_scratch, &E.d_liste, &E.d_dens_orig,
-                    &E.d_rtab, &E.d_itab, &E.d_tprof, &E.d_pairs, &E.d_pair_sums, &E.d_node_aux,
-                    &E.d_forest, &E.d_moff, &E.d_misad, &E.d_mrho, &E.d_task_sort};
+  DevBuf* bufs[] = {&E.d_pos_in, &E.d_mass_in, &E.d_sort, &E.d_x, &E.d_y, &E.d_z, &E.d_m, &E.d_orig, &E.d_rank,
+                    &E.d_box, &E.d_box32, &E.d_cub, &E.d_nei, &E.d_dens, &E.d_group, &E.d_peakflag, &E.d_densg,
+                    &E.d_gpeak, &E.d_goff, &E.d_gmem, &E.d_gmem_rho, &E.d_gmem_rho_pref, &E.d_sad_key,
+                    &E.d_sad_key2, &E.d_sad_val, &E.d_sad_val2, &E.d_sad_cnt, &E.d_sad_keep, &E.d_sad_kpos,
+                    &E.d_flags, &E.d_soff, &E.d_nodes, &E.d_tree_scratch, &E.d_liste, &E.d_dens_orig, &E.d_rtab,
+                    &E.d_itab, &E.d_tprof, &E.d_pairs, &E.d_pair_sums, &E.d_node_aux, &E.d_forest, &E.d_moff,
+                    &E.d_misad, &E.d_mrho, &E.d_task_sort};
   if (E.device >= 0) cudaSetDevice(E.device);
   for (DevBuf* b : bufs) b->release();
   E.h_liste.release(); E.h_dens.release(); E.h_rtab.release(); E.h_itab.release();
@@ -105,6 +104,7 @@ static int run_pipeline(Engine& E, const double* d_pos, const double* d_mass, in
   int rc;
   E.launches = E.cub_calls = E.waves = E.hop_passes = 0;
   cudaStream_t st = E.stream;
+  E.have_groups = false;
   AHOP_CUDA_TRY(cudaEventRecord(E.ev[1], st));
   if ((rc = stage_sort_and_tree(E, d_pos, d_mass))) return rc;
   AHOP_CUDA_TRY(cudaEventRecord(E.ev[2], st));
@@ -134,6 +134,7 @@ static int run_pipeline(Engine& E, const double* d_pos, const double* d_mass, in
     return knn_failed(E) ? AHOP_ELIMIT : AHOP_OK;
   }
   if ((rc = stage_hop_groups(E))) return rc;
+  E.have_groups = true;
   AHOP_CUDA_TRY(cudaEventRecord(E.ev[4], st));
   if (last_stage < 4) return AHOP_OK;
   if ((rc = stage_saddles(E))) return rc;
@@ -513,7 +514,7 @@ __global__ void groups_to_orig_kernel(const int32_t* __restrict__ hop, const int
 
 int ahop_debug_groups(int32_t* hop_target, int32_t* group_id, int32_t* ngroups) {
   Engine& E = engine();
-  if (E.n == 0) { set_error("no result"); return AHOP_ESTATE; }
+  if (E.n == 0 || !E.have_groups) { set_error("no result"); return AHOP_ESTATE; }
   if (ngroups) *ngroups = E.ngroups;
   if (!hop_target && !group_id) return AHOP_OK;
   DevBuf tmp;
@@ -536,8 +537,8 @@ int ahop_debug_saddles(int32_t* nconn, int32_t* offsets, int32_t* isad, double* 
   if (nconn) *nconn = E.nconn;
   cudaStream_t st = E.stream;
   if (offsets) AHOP_CUDA_TRY(cudaMemcpyAsync(offsets, E.d_soff.p, (size_t)(E.ngroups + 1) * 4, cudaMemcpyDeviceToHost, st));
-  if (isad && E.nconn) AHOP_CUDA_TRY(cudaMemcpyAsync(isad, E.d_sisad.p, (size_t)E.nconn * 4, cudaMemcpyDeviceToHost, st));
-  if (rho && E.nconn) AHOP_CUDA_TRY(cudaMemcpyAsync(rho, E.d_srho.p, (size_t)E.nconn * 8, cudaMemcpyDeviceToHost, st));
+  if (isad && E.nconn) AHOP_CUDA_TRY(cudaMemcpyAsync(isad, E.sisad, (size_t)E.nconn * 4, cudaMemcpyDeviceToHost, st));
+  if (rho && E.nconn) AHOP_CUDA_TRY(cudaMemcpyAsync(rho, E.srho, (size_t)E.nconn * 8, cudaMemcpyDeviceToHost, st));
   AHOP_CUDA_TRY(cudaStreamSynchronize(st));
   return AHOP_OK;
 }

@@ -51,6 +51,12 @@ struct CountBuf : DevBuf {
   }
 };
 
+// A part of a buffer.
+struct DevView {
+  void* p = nullptr;
+  template <class T> T* as() const { return static_cast<T*>(p); }
+};
+
 // Growable pinned host buffer (module outputs live here; fast D2H).
 struct HostBuf {
   void* p = nullptr;
@@ -132,12 +138,32 @@ struct Engine {
   int32_t req_store = 0;  // requested via debug API (0 = nhop)
   bool task_profile = false;  // per-task structure-tree profile (debug API)
   bool have_result = false;
+  bool have_groups = false;   // the call's hop targets and groups are there
 
   // inputs / sorted particle arrays
   DevBuf d_pos_in, d_mass_in;            // staging for host inputs
-  DevBuf d_key, d_key2, d_idx, d_idx2;   // Morton keys + permutation
+  // One buffer of 32 bytes per particle: sort keys and permutations, hop targets
+  // and roots as sub-arrays (layout_sort); from the sorted gather to the end of
+  // the kNN, when none of them is in use, it holds the particles as (x, y, z, m)
+  // rows, one sector per gathered particle.
+  DevBuf d_sort;
+  DevView d_key, d_key2, d_idx, d_idx2;  // sort keys (key and key2 are adjacent), sort values and scratch
+  DevView d_hop, d_root;                 // per sorted slot
+  cudaError_t layout_sort() {
+    const size_t N = ((size_t)n + 1 + 63) / 64 * 64;  // n + 1 entries each, 256-byte boundaries
+    const cudaError_t e = d_sort.ensure(32 * N);
+    if (e != cudaSuccess) return e;
+    char* b = d_sort.as<char>();
+    d_key.p = b;
+    d_key2.p = b + 8 * N;
+    d_idx.p = b + 16 * N;
+    d_idx2.p = b + 20 * N;
+    d_hop.p = b + 24 * N;
+    d_root.p = b + 28 * N;
+    return cudaSuccess;
+  }
+  double4* rows() const { return d_sort.as<double4>(); }
   DevBuf d_x, d_y, d_z, d_m;             // sorted SoA
-  DevBuf d_p4;                           // the same as (x, y, z, m) rows: one sector per gathered particle
   DevBuf d_orig;                         // orig index (0-based) per sorted slot
   DevBuf d_rank;                         // sorted slot per orig index
   DevBuf d_box;                          // AABBs of all levels (6 doubles each)
@@ -149,10 +175,9 @@ struct Engine {
 
   // kNN / density
   DevBuf d_nei;                          // [n][nstore] sorted-slot neighbour ids
-  DevBuf d_coll;                         // collected slots and counts of a chunk of query leaves
   DevBuf d_dens;                         // density in sorted order
   // hop / groups
-  DevBuf d_hop, d_root, d_group;         // per sorted slot
+  DevBuf d_group;                        // per sorted slot
   DevBuf d_peakflag;                     // per orig index
   int32_t ngroups = 0;
   CountBuf d_densg;                        // [ngroups+1] peak density per group
@@ -165,7 +190,9 @@ struct Engine {
   // saddles
   CountBuf d_sad_key, d_sad_key2, d_sad_val, d_sad_val2, d_sad_cnt, d_sad_keep, d_sad_kpos;
   DevBuf d_flags;                        // small device error/status flags
-  CountBuf d_soff, d_sisad, d_srho;        // final CSR
+  CountBuf d_soff;                       // final CSR: row offsets,
+  int32_t* sisad = nullptr;              // neighbour groups (inside d_sad_key2)
+  double* srho = nullptr;                // and saddles (inside d_sad_key)
   int32_t nconn = 0;
   // nodes
   CountBuf d_nodes;                        // NodeRec[nnodesmax+1]
@@ -181,7 +208,7 @@ struct Engine {
   CountBuf d_node_aux;                     // per node: pair range, posref
   int32_t nnodes = 0;
   DevBuf d_liste;                        // [n] node id per ORIG particle (1-based), 0 none
-  DevBuf d_dens_orig;                    // [n] density in ORIG order
+  DevBuf d_dens_orig;                    // [n] density in ORIG order; before that the kNN's collected slots
   CountBuf d_rtab, d_itab;                 // exported tables
 
   // host copies (module outputs), pinned

@@ -281,8 +281,8 @@ int build_saddle_forest(Engine& E) {
   ForestArgs F;
   F.ng = ng;
   F.soff = E.d_soff.as<int32_t>();
-  F.sisad = E.d_sisad.as<int32_t>();
-  F.srho = E.d_srho.as<double>();
+  F.sisad = E.sisad;
+  F.srho = E.srho;
   F.comp = reinterpret_cast<int32_t*>(take(G * 4));
   F.cur = reinterpret_cast<int32_t*>(take(G * 4));
   F.gbest = reinterpret_cast<int32_t*>(take(G * 4));

@@ -116,8 +116,6 @@ int stage_hop_groups(Engine& E) {
   cudaStream_t st = E.stream;
   const int T = 256;
   const unsigned grid = (unsigned)((n + T - 1) / T);
-  AHOP_CUDA_TRY(E.d_hop.ensure(n * 4));
-  AHOP_CUDA_TRY(E.d_root.ensure(n * 4));
   AHOP_CUDA_TRY(E.d_group.ensure(n * 4));
   AHOP_CUDA_TRY(E.d_peakflag.ensure((n + 1) * 4));
   int32_t* hop = E.d_hop.as<int32_t>();
@@ -138,7 +136,6 @@ int stage_hop_groups(Engine& E) {
   peak_flag_kernel<<<grid, T, 0, st>>>(hop, E.d_orig.as<int32_t>(), n, flag);
   AHOP_CUDA_TRY(cudaGetLastError());
   AHOP_CUDA_TRY(cudaMemsetAsync(flag + n, 0, 4, st));
-  AHOP_CUDA_TRY(E.d_idx.ensure((n + 1) * 4));
   int32_t* scan = E.d_idx.as<int32_t>();  // sort scratch no longer needed
   size_t tmp = 0;
   cub::DeviceScan::ExclusiveSum(nullptr, tmp, flag, scan, (int)(n + 1), st);
@@ -174,9 +171,6 @@ int stage_hop_groups(Engine& E) {
     AHOP_CUDA_TRY(cub::DeviceScan::ExclusiveSum(E.d_cub.p, t2, gcount, E.d_goff.as<int32_t>(), ng + 2, st));
   }
   // member CSR in (group asc, particle index desc)
-  AHOP_CUDA_TRY(E.d_key.ensure(n * 8));
-  AHOP_CUDA_TRY(E.d_key2.ensure(n * 8));
-  AHOP_CUDA_TRY(E.d_idx2.ensure(n * 4));
   AHOP_CUDA_TRY(E.d_gmem.ensure(n * 4));
   E.launches++;
   const int ob = bits_for(n);  // 2^ob > n > every particle index

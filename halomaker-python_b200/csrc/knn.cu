@@ -57,13 +57,12 @@ __global__ void morton_kernel(const double* __restrict__ pos, int64_t n, double 
 }
 
 __global__ void gather_sorted_kernel(const double* __restrict__ pos, const double* __restrict__ mass,
-                                     const int32_t* __restrict__ idx, int64_t n, double* __restrict__ x,
+                                     const int32_t* __restrict__ orig, int64_t n, double* __restrict__ x,
                                      double* __restrict__ y, double* __restrict__ z, double* __restrict__ m,
-                                     double4* __restrict__ p4, int32_t* __restrict__ orig,
-                                     int32_t* __restrict__ rank) {
+                                     double4* __restrict__ p4, int32_t* __restrict__ rank) {
   int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (s >= n) return;
-  int32_t o = idx[s];
+  int32_t o = orig[s];
   const double px = pos[3 * (int64_t)o + 0], py = pos[3 * (int64_t)o + 1], pz = pos[3 * (int64_t)o + 2];
   const double pm = mass[o];
   x[s] = px;
@@ -71,7 +70,6 @@ __global__ void gather_sorted_kernel(const double* __restrict__ pos, const doubl
   z[s] = pz;
   m[s] = pm;
   p4[s] = make_double4(px, py, pz, pm);
-  orig[s] = o;
   rank[o] = (int32_t)s;
 }
 
@@ -133,15 +131,11 @@ int stage_sort_and_tree(Engine& E, const double* d_pos, const double* d_mass) {
   const int64_t n = E.n;
   const Params& P = E.prm;
   cudaStream_t st = E.stream;
-  AHOP_CUDA_TRY(E.d_key.ensure(n * 8));
-  AHOP_CUDA_TRY(E.d_key2.ensure(n * 8));
-  AHOP_CUDA_TRY(E.d_idx.ensure(n * 4));
-  AHOP_CUDA_TRY(E.d_idx2.ensure(n * 4));
+  AHOP_CUDA_TRY(E.layout_sort());
   AHOP_CUDA_TRY(E.d_x.ensure(n * 8));
   AHOP_CUDA_TRY(E.d_y.ensure(n * 8));
   AHOP_CUDA_TRY(E.d_z.ensure(n * 8));
   AHOP_CUDA_TRY(E.d_m.ensure(n * 8));
-  AHOP_CUDA_TRY(E.d_p4.ensure(n * 32));
   AHOP_CUDA_TRY(E.d_orig.ensure(n * 4));
   AHOP_CUDA_TRY(E.d_rank.ensure(n * 4));
   const int T = 256;
@@ -157,20 +151,21 @@ int stage_sort_and_tree(Engine& E, const double* d_pos, const double* d_mass) {
   size_t tmp = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, tmp, E.d_key.as<unsigned long long>(),
                                   E.d_key2.as<unsigned long long>(), E.d_idx.as<int32_t>(),
-                                  E.d_idx2.as<int32_t>(), (int)n, 0, 63, st);
+                                  E.d_orig.as<int32_t>(), (int)n, 0, 63, st);
   AHOP_CUDA_TRY(E.d_cub.ensure(tmp));
   E.cub_calls++;
   AHOP_CUDA_TRY(cub::DeviceRadixSort::SortPairs(E.d_cub.p, tmp, E.d_key.as<unsigned long long>(),
                                                 E.d_key2.as<unsigned long long>(), E.d_idx.as<int32_t>(),
-                                                E.d_idx2.as<int32_t>(), (int)n, 0, 63, st));
+                                                E.d_orig.as<int32_t>(), (int)n, 0, 63, st));
   E.launches++;
   if (E.mass_pending) {  // host path: the masses were uploaded on the copy stream
     AHOP_CUDA_TRY(cudaStreamWaitEvent(st, E.ev_mass, 0));
     E.mass_pending = false;
   }
-  gather_sorted_kernel<<<grid, T, 0, st>>>(d_pos, d_mass, E.d_idx2.as<int32_t>(), n, E.d_x.as<double>(),
-                                           E.d_y.as<double>(), E.d_z.as<double>(), E.d_m.as<double>(),
-                                           E.d_p4.as<double4>(), E.d_orig.as<int32_t>(), E.d_rank.as<int32_t>());
+  // the keys and the permutation's first copy give way to the rows
+  gather_sorted_kernel<<<grid, T, 0, st>>>(d_pos, d_mass, E.d_orig.as<int32_t>(), n, E.d_x.as<double>(),
+                                           E.d_y.as<double>(), E.d_z.as<double>(), E.d_m.as<double>(), E.rows(),
+                                           E.d_rank.as<int32_t>());
   AHOP_CUDA_TRY(cudaGetLastError());
   // levels
   int64_t cnt = (n + kLeaf - 1) / kLeaf;
@@ -1266,7 +1261,7 @@ int stage_knn_density(Engine& E) {
   AHOP_CUDA_TRY(E.d_nei.ensure((size_t)n * E.nstore * 4));
   AHOP_CUDA_TRY(E.d_dens.ensure(n * 8));
   KnnArgs A;
-  A.p4 = E.d_p4.as<double4>();
+  A.p4 = E.rows();
   A.m = E.d_m.as<double>();
   A.orig = E.d_orig.as<int32_t>();
   A.box = E.d_box.as<double>();
@@ -1317,13 +1312,13 @@ int stage_knn_density(Engine& E) {
   if (per_sm < 1) per_sm = 1;
   const int64_t nleaf = E.lev_cnt[0];
   const int64_t chunk = std::min<int64_t>(nleaf, kChunkLeaves);
-  AHOP_CUDA_TRY(E.d_coll.ensure((size_t)chunk * (kCollect * 32 * 4 + 32 * 4 + 32)));
-  A.coll = E.d_coll.as<int32_t>();
+  const bool all = n <= kPerQueryMax;
+  if (!all) AHOP_CUDA_TRY(E.d_dens_orig.ensure((size_t)chunk * (kCollect * 32 * 4 + 32 * 4 + 32)));
+  A.coll = E.d_dens_orig.as<int32_t>();
   A.lost = A.coll + (size_t)chunk * kCollect * 32;
   A.ccnt = reinterpret_cast<uint8_t*>(A.lost + (size_t)chunk * 32);
   A.nlost = A.next + 1;
   AHOP_CUDA_TRY(cudaEventRecord(E.ev[9], E.stream));
-  const bool all = n <= kPerQueryMax;
   if (all) {
     const unsigned g = (unsigned)((n + kFinWarps - 1) / kFinWarps);
     if (nv32) knn_query_kernel<32, true><<<g, kFinWarps * 32, 0, E.stream>>>(A);

@@ -2324,8 +2324,6 @@ int stage_nodes(Engine& E) {
   if (nact > 0) {
     // one radix sort of (group, density rounded to float), then exact order
     // inside runs of equal keys (member_rho_keys_kernel)
-    AHOP_CUDA_TRY(E.d_key.ensure((size_t)nact * 8));
-    AHOP_CUDA_TRY(E.d_key2.ensure((size_t)nact * 8));
     unsigned long long* k0 = E.d_key.as<unsigned long long>();
     unsigned long long* k1 = E.d_key2.as<unsigned long long>();
     const unsigned gm = (unsigned)((nact + T - 1) / T);
@@ -2776,8 +2774,7 @@ int stage_nodes(Engine& E) {
   AHOP_CUDA_TRY(E.d_rtab.ensure((size_t)(nn > 0 ? nn : 1) * 64));
   AHOP_CUDA_TRY(E.d_itab.ensure((size_t)(nn > 0 ? nn : 1) * 24));
   if (nn > 0) {
-    AHOP_CUDA_TRY(E.d_idx2.ensure((size_t)(nn + 1) * 4 * 2));
-    int32_t* new_to_old = E.d_idx2.as<int32_t>();
+    int32_t* new_to_old = E.d_key.as<int32_t>();  // key and key2: 16 bytes per particle, nn is below 2 n
     int32_t* o2n = new_to_old + nn + 1;
     E.launches++;
     iota_kernel<<<(unsigned)((nn + T - 1) / T), T, 0, st>>>(new_to_old, nn, 1);

@@ -117,8 +117,6 @@ int stage_saddles(Engine& E) {
   const unsigned grid = (unsigned)((n + T - 1) / T);
   const int32_t ng = E.ngroups;
   // per-particle link counts and offsets
-  AHOP_CUDA_TRY(E.d_idx2.ensure((n + 1) * 4));
-  AHOP_CUDA_TRY(E.d_idx.ensure((n + 1) * 4));
   int32_t* cnt = E.d_idx2.as<int32_t>();
   int32_t* off = E.d_idx.as<int32_t>();
   AHOP_CUDA_TRY(E.d_flags.ensure(512));
@@ -150,12 +148,13 @@ int stage_saddles(Engine& E) {
   AHOP_CUDA_TRY(E.d_sad_val.ensure(nl * 8));
   AHOP_CUDA_TRY(E.d_sad_val2.ensure(nl * 8));
   AHOP_CUDA_TRY(E.d_soff.ensure((size_t)(ng + 2) * 4));
+  // the rows end up where the link keys are no longer needed
+  E.srho = E.d_sad_key.as<double>();
+  E.sisad = E.d_sad_key2.as<int32_t>() + nl;
   E.nconn = 0;
   E.h_scalars[Engine::kHostScalars - 2] = 0;
   if (nlink == 0) {
     AHOP_CUDA_TRY(cudaMemsetAsync(E.d_soff.p, 0, (size_t)(ng + 2) * 4, st));
-    AHOP_CUDA_TRY(E.d_sisad.ensure(4));
-    AHOP_CUDA_TRY(E.d_srho.ensure(8));
     return AHOP_OK;
   }
   int gb = 1;
@@ -209,8 +208,6 @@ int stage_saddles(Engine& E) {
   AHOP_CUDA_TRY(cub::DeviceScan::ExclusiveSum(E.d_cub.p, tmp, keep, kpos, nlink + 1, st));
   // read by saddles_counted after the next synchronisation
   AHOP_CUDA_TRY(cudaMemcpyAsync(E.h_scalars + Engine::kHostScalars - 2, kpos + nlink, 4, cudaMemcpyDeviceToHost, st));
-  AHOP_CUDA_TRY(E.d_sisad.ensure(nl * 4));
-  AHOP_CUDA_TRY(E.d_srho.ensure(nl * 8));
   // row offsets over groups: soff[g-1] .. soff[g] for group g (rowcnt index g)
   tmp = 0;
   cub::DeviceScan::ExclusiveSum(nullptr, tmp, rowcnt + 1, E.d_soff.as<int32_t>(), ng + 1, st);
@@ -225,13 +222,13 @@ int stage_saddles(Engine& E) {
   AHOP_CUDA_TRY(cudaGetLastError());
   // segmented sort by value descending within each row (payload: neighbour id)
   tmp = 0;
-  cub::DeviceSegmentedSort::StableSortPairsDescending(nullptr, tmp, E.d_sad_val.as<double>(), E.d_srho.as<double>(),
-                                                      isad, E.d_sisad.as<int32_t>(), nlink, ng,
+  cub::DeviceSegmentedSort::StableSortPairsDescending(nullptr, tmp, E.d_sad_val.as<double>(), E.srho,
+                                                      isad, E.sisad, nlink, ng,
                                                       E.d_soff.as<int32_t>(), E.d_soff.as<int32_t>() + 1, st);
   AHOP_CUDA_TRY(E.d_cub.ensure(tmp));
   E.cub_calls++;
   AHOP_CUDA_TRY(cub::DeviceSegmentedSort::StableSortPairsDescending(
-      E.d_cub.p, tmp, E.d_sad_val.as<double>(), E.d_srho.as<double>(), isad, E.d_sisad.as<int32_t>(), nlink, ng,
+      E.d_cub.p, tmp, E.d_sad_val.as<double>(), E.srho, isad, E.sisad, nlink, ng,
       E.d_soff.as<int32_t>(), E.d_soff.as<int32_t>() + 1, st));
   return AHOP_OK;
 }

@@ -67,6 +67,28 @@ def test_growth_takes_no_more():
     assert grown <= alone + PAGES, (grown, alone)
 
 
+def test_bytes_per_particle():
+    # without groups, by array: inputs 32, sort keys, permutations, hop targets
+    # and roots 32, sorted x, y, z, m 32, index and rank 8, boxes 80 per 31,
+    # neighbours 64, density in both orders 16, group, peak flag, members and
+    # node ids 16, the radix sort's second copy of keys and values 12; from 8.4M
+    # particles on the kNN's collected slots are no larger (1.65 GB)
+    _held([1000])
+    small = _held([9000000])[0]
+    large = _held([18000000])[0]
+    assert large - small <= 9000000 * 214.6 + PAGES, (large - small) / 9e6
+    assert large <= 18000000 * 214.6 + 1.66e9 + PAGES, large
+
+
+def test_groups_view_needs_its_stage():
+    from ahop_b200 import _lib, finder
+    pos = _uniform(5000)
+    finder.configure(5000)
+    finder.run_stages(pos, np.full(5000, 2e-4), last_stage=2)
+    hop = np.zeros(5000, np.int32)
+    assert _lib.lib().ahop_debug_groups(hop.ctypes.data, hop.ctypes.data, None) == 4  # ESTATE
+
+
 def test_growth_where_just_enough_is_free():
     import torch
     _held([1000])
