@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(256) pack_kernel(const double* __restrict__ po
 // (n, 3) positions and the masses); the lists of a warp's 32 particles are read
 // as rows of 128 bytes and turned in shared memory.
 // 2,097,152 particles with 32 neighbours, ms: forward 0.87 (L2 at 87 % of its
-// rate) -> 0.45, backward 2.39 -> 1.08 (latency of the gathers, 24 warps per
+// rate) -> 0.44, backward 2.39 -> 1.19 (latency of the gathers, 24 warps per
 // SM; the atomics alone were 3 x 32 sectors per neighbour and warp).
 constexpr int kAB = 128;                   // threads per block
 constexpr int64_t kPackMin = 32768;        // below, the extra launch costs more than it saves
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(kAB, 6) density_adjoint_kernel(AdjArgs A, cons
 // shared memory.  Positions relative to the member at centre[h] (the densest)
 // with the strict min-image rule.  Bound by the FP64 pipe, 17 operations per
 // ordered pair; the partners are split so that a few large halos still fill
-// the device (500 halos, 217M pairs: backward pass 3.0 -> 0.9 ms).  A row tile
+// the device (500 halos, 217M pairs: backward pass 3.0 -> 0.75 ms).  A row tile
 // with one item is added to gpos here, the others leave their sums in part for
 // epot_grad_fold_kernel, which adds them in item order.
 constexpr int kGT = 256;              // rows per item and partner tile

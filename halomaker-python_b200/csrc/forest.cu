@@ -45,7 +45,7 @@ struct ForestArgs {
   unsigned long long* bk;  // [ng+1] smallest edge key at that weight
   unsigned long long* fkey;  // [ng] forest edges: lower id << 32 | higher id
   double* fw;                // [ng] forest edge saddles
-  int32_t* ctr;            // [0] forest edges, [1] hooks this round, [2] jump not finished
+  int32_t* ctr;            // [0] forest edges, [1] hooks this round, [2] jump not finished, [3] rounds (one block)
 };
 
 __device__ __forceinline__ unsigned long long edge_key(int32_t g, int32_t h) {

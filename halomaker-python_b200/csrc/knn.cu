@@ -426,7 +426,7 @@ __global__ void leaf_box32_kernel(const double* __restrict__ box, int64_t nbox, 
 // Bound by instruction issue: 1,620 warp instructions per query (8M-particle
 // clustered box; one warp per query with a list in registers took 3,751, most
 // of them in visiting each query's own leaves and inserting one by one), 16.7M
-// particles in 36.3 ms against 87.3, 2M in 4.7 against 13.4.
+// particles in 35.9 ms against 87.3, 2M in 4.65 against 13.1.
 // The main path works on a query leaf's 32 particles at once, lane = query, so
 // every per-query step costs 1/32 of a warp instruction per query and the
 // particles of a candidate leaf are read from shared memory by all 32 queries.
@@ -440,17 +440,19 @@ constexpr int kFinBlocks = 5;      // finish: blocks per SM
 constexpr int kLostBlocks = 16;    // blocks per SM for the queries left over: usually few, at times whole chunks
 constexpr int kBatch = 256;        // candidate leaves sorted and counted at a time
 constexpr int kVisMax = 160;       // counted leaves per query leaf, three times the mean; beyond, a warp for each
-                                   // of the 32 queries is as cheap and ends sooner (262,144 particles: 1.15-1.29
-                                   // ms at 160, 1.32-1.59 at 352)
+                                   // of the 32 queries is as cheap and ends sooner (262,144 particles, three
+                                   // boxes: 0.95-1.11 ms at 160, 0.94-1.24 at 352; 2M and 16.7M: the same)
 // Nodes opened and candidate leaves listed per query leaf, far above the means
 // (about 40 and 125): a leaf strung over distant clumps would otherwise keep
-// one warp long after the others are done (without the limits 2.5 of 9.5
-// Mcycles at 2M particles; 16.7M: 43.3 -> 36.3 ms, 262,144: 1.35 -> 0.99).
+// one warp long after the others are done (three boxes each, without the limits
+// and with: 262,144 particles 1.13-1.40 ms, 0.95-1.11; 2M 5.2-6.1, 4.65; 16.7M
+// 41-51, 35.9).
 constexpr int kNodeMax = 256, kCandMax = 768;
 // Up to here every query gets a warp of its own: a set of fewer query leaves
 // than resident warps (3,552) takes as long as its slowest leaf.  Measured
-// (ms, per query | per lane): 5,003 particles 0.08 | 0.48, 40,000 0.33 | 0.60,
-// 70,001 0.55 | 0.75, 131,072 1.02 | 0.80, 262,144 2.04 | 1.15.
+// (ms, per query | per lane, means of three boxes): 20,000 particles 0.20 |
+// 0.50, 70,001 0.56 | 0.62, 98,304 0.76 | 0.76, 131,072 1.02 | 0.85, 262,144
+// 2.01 | 1.05.
 constexpr int kPerQueryMax = 98304;
 constexpr int kTravStack = 192;    // traversal stack: at most 31 nodes waiting per level and 32 at the last
 constexpr int kTile = 64;          // particles staged: up to 31 left over and one leaf

@@ -2776,9 +2776,6 @@ int stage_nodes(Engine& E) {
   if (nn > 0) {
     int32_t* new_to_old = E.d_key.as<int32_t>();  // key and key2: 16 bytes per particle, nn is below 2 n
     int32_t* o2n = new_to_old + nn + 1;
-    E.launches++;
-    iota_kernel<<<(unsigned)((nn + T - 1) / T), T, 0, st>>>(new_to_old, nn, 1);
-    AHOP_CUDA_TRY(cudaGetLastError());
     if (nn <= kRankNodes) {
       AHOP_CUDA_TRY(cudaMemsetAsync(o2n, 0, (size_t)(nn + 1) * 4, st));  // ranks, then the inverse
       const unsigned nb = (unsigned)((nn + 255) / 256);
@@ -2787,6 +2784,9 @@ int stage_nodes(Engine& E) {
       node_place_kernel<<<nb, 256, 0, st>>>(o2n, nn, new_to_old);
       AHOP_CUDA_TRY(cudaGetLastError());
     } else {
+      E.launches++;
+      iota_kernel<<<(unsigned)((nn + T - 1) / T), T, 0, st>>>(new_to_old, nn, 1);
+      AHOP_CUDA_TRY(cudaGetLastError());
       size_t tmp = 0;
       NodeLess less{A.node};
       cub::DeviceMergeSort::SortKeys(nullptr, tmp, new_to_old, nn, less, st);

@@ -36,7 +36,6 @@
 #include <cstring>
 #include <mutex>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -357,8 +356,8 @@ extern "C" int ahop_ramses_open(const char* const* paths, int32_t nfiles, const 
     std::vector<std::thread> readers;
     try {
       for (int t = 1; t < nr; ++t) readers.emplace_back(read_pieces, std::ref(S), std::ref(J), dev, t);
-    } catch (const std::system_error&) {
-      // fewer threads: the pieces are shared out as they are taken
+    } catch (...) {
+      // no thread or no memory for one: fewer readers, the pieces are shared out as they are taken
     }
     read_pieces(S, J, dev, 0);
     for (auto& t : readers) t.join();

@@ -78,7 +78,7 @@ typedef struct {
   /* parts of `nodes`: per-group density-sorted members and running sums,
    * root level, task waves, membership + renumbering + tables */
   float nodes_prep, nodes_root, nodes_waves, nodes_order;
-  int32_t kernel_launches, cub_calls, tree_waves, hop_passes;
+  int32_t kernel_launches, cub_calls, tree_waves, hop_passes; /* hop_passes: 1, all chains end in one launch */
 } AhopTimings;
 
 const char* ahop_last_error(void);
