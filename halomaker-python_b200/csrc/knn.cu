@@ -397,8 +397,9 @@ __device__ __forceinline__ void finish_query(const KnnArgs& A, const WarpList& L
 // on some axis (the boxes' padding, for one); the reference's distance is 0
 // there, which only the per-query search takes, so beyond 1e-9 of the box it
 // is +inf (a particle outside the box, and the leaves across the box from it),
-// as where FP32 coordinates or distances would be too coarse (inbox = 0, or
-// particles outside [-L, L]).
+// as where FP32 coordinates are too coarse (particles outside [-L, L]) or squares
+// leave the range of floats (inbox = 0: L above 1e15, or below 1e-8, where the
+// 2^-149 of a subnormal square, 6e-23 as a distance, exceeds eabs2 = 2^-45 L).
 __global__ void leaf_box32_kernel(const double* __restrict__ box, int64_t nbox, double Lx, double Ly, double Lz,
                                   int inbox, float4* __restrict__ out) {
   const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -1273,7 +1274,7 @@ int stage_knn_density(Engine& E) {
   const double Lmin = std::min(P.xlong, std::min(P.ylong, P.zlong)), Lmax = std::max(P.xlong, std::max(P.ylong, P.zlong));
   E.launches++;
   leaf_box32_kernel<<<(unsigned)((nbox + 255) / 256), 256, 0, E.stream>>>(
-      A.box, nbox, P.xlong, P.ylong, P.zlong, Lmax < 1e15 && Lmin > 1e-15, E.d_box32.as<float4>());
+      A.box, nbox, P.xlong, P.ylong, P.zlong, Lmax < 1e15 && Lmin > 1e-8, E.d_box32.as<float4>());
   AHOP_CUDA_TRY(cudaGetLastError());
   for (int l = 0; l < kMaxLevels; ++l) { A.lev_off[l] = E.lev_off[l]; A.lev_cnt[l] = E.lev_cnt[l]; }
   A.nlev = E.nlev;
