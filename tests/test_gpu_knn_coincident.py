@@ -40,3 +40,24 @@ def test_coincident_rows(n, nv):
         first = mem[:nv + 1]  # in index order
         for i in mem:
             assert np.array_equal(rows[i], first[first != i][:nv]), (c, len(mem), i)
+
+
+@pytest.mark.parametrize("n,nmemb", [(20000, 20), (20000, 100), (120000, 20)])
+def test_whole_finder(n, nmemb):
+    # three clumps of coincident particles (infinite density) inside one dense
+    # cloud, linked to its groups by finite saddles
+    import oracle
+    from ahop_b200 import finder
+    rng = np.random.default_rng(3)
+    pos = np.concatenate([rng.random((n - 9000, 3)) - 0.5, 0.01 * rng.normal(size=(9000, 3)) + 0.1])
+    pos[:500] = [0.1, 0.1, 0.1]
+    pos[500:540] = [0.112, 0.1, 0.1]
+    pos[540:575] = [0.1, 0.115, 0.1]
+    pos = pos[rng.permutation(n)]
+    mass = np.full(n, 1.0 / n)
+    finder.configure(n, nmembthresh=nmemb)
+    got = finder.run(pos, mass)
+    ref = oracle.run(pos, mass, oracle.default_params(n, nmembthresh=nmemb))
+    assert got["ngroups"] == ref["ngroups"] and got["nnodes"] == ref["nnodes"]
+    for f in ("density", "liste_parts", "integer_table", "real_table"):
+        assert np.array_equal(got[f], ref[f]), f
