@@ -66,7 +66,9 @@ static int with_room(Engine& E, F&& compute) {
   int rc = compute();
   if (rc != AHOP_ENOMEM) return rc;
   cudaGetLastError();
-  for (cudaStream_t s : {E.stream, E.stream2, E.stream_copy}) AHOP_CUDA_TRY(cudaStreamSynchronize(s));
+  AHOP_CUDA_TRY(cudaStreamSynchronize(E.stream));
+  if (E.stream2) AHOP_CUDA_TRY(cudaStreamSynchronize(E.stream2));
+  if (E.stream_copy) AHOP_CUDA_TRY(cudaStreamSynchronize(E.stream_copy));
   release_device(E);
   exact_buffers = true;
   rc = compute();
