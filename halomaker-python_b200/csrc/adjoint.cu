@@ -81,8 +81,9 @@ __global__ void __launch_bounds__(256) pack_kernel(const double* __restrict__ po
 // (n, 3) positions and the masses); the lists of a warp's 32 particles are read
 // as rows of 128 bytes and turned in shared memory.
 // 2,097,152 particles with 32 neighbours, ms: forward 0.87 (L2 at 87 % of its
-// rate) -> 0.44, backward 2.39 -> 1.19 (latency of the gathers, 24 warps per
-// SM; the atomics alone were 3 x 32 sectors per neighbour and warp).
+// rate) -> 0.44, backward 2.39 -> 1.13 (latency of the gathers, 28 warps per
+// SM: 24 with four neighbours unrolled 1.19, 32 spill, 1.26; the atomics alone
+// were 3 x 32 sectors per neighbour and warp).
 constexpr int kAB = 128;                   // threads per block
 constexpr int64_t kPackMin = 32768;        // below, the extra launch costs more than it saves
 
@@ -150,7 +151,7 @@ __device__ __forceinline__ void scatter_add(double* __restrict__ gpos, int64_t j
 }
 
 template <bool kPacked>
-__global__ void __launch_bounds__(kAB, 6) density_adjoint_kernel(AdjArgs A, const double* __restrict__ gdens,
+__global__ void __launch_bounds__(kAB, 7) density_adjoint_kernel(AdjArgs A, const double* __restrict__ gdens,
                                                                  double* __restrict__ gpos) {
   __shared__ int32_t s_tile[kAB / 32][32][33];
   __shared__ double s_v[kAB / 32][96];
@@ -177,15 +178,14 @@ __global__ void __launch_bounds__(kAB, 6) density_adjoint_kernel(AdjArgs A, cons
   for (int k0 = 0; k0 < A.nv - 1; k0 += 32) {
     stage_lists(A, i0, k0, lane, tile);
     const int m = min(32, A.nv - 1 - k0);
-#pragma unroll 4
+#pragma unroll 1  // unrolled, the divisions' slow paths spill
     for (int k = 0; k < m; ++k) {
       const int64_t j = act ? tile[lane][k] : 0;
       const double4 q = particle<kPacked>(A, j);
       const double dx = pdelta(me.x, q.x, A.Lx), dy = pdelta(me.y, q.y, A.Ly), dz = pdelta(me.z, q.z, A.Lz);
       const double d2 = dx * dx + dy * dy + dz * dz;
       // one rounding each: through a reciprocal root and 1 / r a pair's term is
-      // off by up to 8.5 half units in the last place instead of 3 (1.62 ms
-      // for 2,097,152 particles, forward and backward, against 1.69)
+      // off by up to 8.5 half units in the last place instead of 3, and no faster
       const double d = sqrt(d2);
       const double u = d / r;
       S += q.w * spline(u);
