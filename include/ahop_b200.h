@@ -255,6 +255,8 @@ typedef struct {
 } AhopRamsesCounts;
 int ahop_ramses_open(const char* const* paths, int32_t nfiles, const AhopRamsesParams* p, AhopRamsesCounts* out);
 int ahop_ramses_decode_device(double* d_pos, double* d_vel, double* d_mass, int64_t* d_source_pid, void* stream);
+/* Closes the files; the staging stays for the next ones (64 MB pinned, up to
+ * 1 GB on the device) until ahop_release_device_memory. */
 int ahop_ramses_close(void);
 
 /* ---- batched halo properties ------------------------------------------------

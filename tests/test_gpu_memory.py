@@ -94,7 +94,10 @@ def test_growth_where_just_enough_is_free():
     _held([1000])
     alone, want = _held([3300000], _clustered)
     free = _release()
-    block = torch.empty(free - alone - PAGES, dtype=torch.uint8, device="cuda")
+    try:
+        block = torch.empty(free - alone - PAGES, dtype=torch.uint8, device="cuda")
+    except torch.OutOfMemoryError:
+        pytest.skip("another process took device memory meanwhile")
     try:
         _run(_clustered(2900000))
         got = _run(_clustered(3300000))
